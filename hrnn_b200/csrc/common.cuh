@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 
 #include "../../include/hrnn_capi.h"
 
@@ -72,17 +73,25 @@ __device__ __forceinline__ float sq_step(float acc, float t, bool fused) {
 // One thread, any dim: restates the dispatch of space_l2.h:214-238.
 __device__ inline float l2_thread(const float* __restrict__ a, const float* __restrict__ b,
                                   uint32_t d, int lanes, int fused) {
-    auto simd = [&](uint32_t len, int L) {
-        float acc[16];
+    // accumulator indexes known at compile time, so they stay in registers
+    auto simd_n = [&](uint32_t len, auto lanes_c) {
+        constexpr int L = decltype(lanes_c)::value;
+        float acc[L];
 #pragma unroll
-        for (int l = 0; l < 16; ++l) acc[l] = 0.f;
-        for (uint32_t e = 0; e < len; ++e) {
-            int l = (int)(e % (uint32_t)L);
-            acc[l] = sq_step(acc[l], a[e] - b[e], fused & 1);
+        for (int l = 0; l < L; ++l) acc[l] = 0.f;
+        for (uint32_t e = 0; e < len; e += L) {  // len is a multiple of L
+#pragma unroll
+            for (int l = 0; l < L; ++l) acc[l] = sq_step(acc[l], a[e + l] - b[e + l], fused & 1);
         }
         float r = acc[0];
+#pragma unroll
         for (int l = 1; l < L; ++l) r = __fadd_rn(r, acc[l]);
         return r;
+    };
+    auto simd = [&](uint32_t len, int L) {
+        if (L == 16) return simd_n(len, std::integral_constant<int, 16>{});
+        if (L == 8) return simd_n(len, std::integral_constant<int, 8>{});
+        return simd_n(len, std::integral_constant<int, 4>{});
     };
     auto scalar = [&](uint32_t off, uint32_t len) {
         float r = 0.f;

@@ -74,8 +74,11 @@ namespace {
 
 // DM: distance mode of beam.cuh (0/1 exact FP32 unfused/fused, 2 BF16 rows, 3
 // INT8 rows against the INT8-quantised query).
-template <int DM>
-__global__ void __launch_bounds__(128) k_phase_a(DevView v, const float* __restrict__ Q, uint32_t nq,
+// T: warps per query.  1: a warp of its own for each query.  kTeamWarps (exact forms):
+// the block's warps search for one query (beam_search_team), for batches too small to
+// fill the device.
+template <int DM, int RK, int T>
+__global__ void __launch_bounds__(T == 1 ? 128 : 32 * T, T == 1 ? 4 : RK == 64 || RK == kRows4 ? 3 : 2) k_phase_a(DevView v, const float* __restrict__ Q, uint32_t nq,
                                                  const uint32_t* __restrict__ qm, const uint32_t* __restrict__ qef,
                                                  uint32_t efc, uint32_t vc, uint32_t mmax,
                                                  uint32_t* __restrict__ prox, uint32_t* __restrict__ nprox,
@@ -94,37 +97,56 @@ __global__ void __launch_bounds__(128) k_phase_a(DevView v, const float* __restr
     // the next query as soon as it finishes one.
     extern __shared__ char smem_raw[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    WarpSmem s = carve(smem_raw + (size_t)w * warp_smem_bytes(v.dim, efc, vc), v.dim, efc, vc);
+    const uint32_t ut = T == 1 ? lane : threadIdx.x, un = 32 * T;  // thread within the query's warps
+    WarpSmem s = carve(smem_raw + (T == 1 ? (size_t)w * warp_smem_bytes(v.dim, efc, vc) : 0), v.dim, efc, vc);
     unsigned long long c_dist = 0, c_exp = 0;
     if (nq_dev) nq = min(nq, *nq_dev);
     for (;;) {
         uint32_t j = 0;
-        if (lane == 0) j = atomicAdd(next_q, 1u);
-        j = __shfl_sync(0xFFFFFFFFu, j, 0);
+        if (ut == 0) j = atomicAdd(next_q, 1u);
+        if constexpr (T == 1) {
+            j = __shfl_sync(0xFFFFFFFFu, j, 0);
+        } else {
+            if (ut == 0) s.apos[0] = j;
+            __syncthreads();
+            j = s.apos[0];
+            __syncthreads();
+        }
         if (j >= nq) break;
         const uint32_t qi = qlist ? qlist[j] : j;
         const uint32_t m = m_over ? m_over : qm[qi];
         const uint32_t EF = max(ef_over ? ef_over : qef[qi], m);
         if (v.n == 0 || m == 0) {
-            if (lane == 0) nprox[qi] = 0;
+            if (ut == 0) nprox[qi] = 0;
             continue;
         }
-        for (uint32_t i = lane; i < v.dim; i += 32) s.q[i] = Q[(size_t)qi * v.dim + i];
-        __syncwarp();
+        for (uint32_t i = ut; i < v.dim; i += un) s.q[i] = Q[(size_t)qi * v.dim + i];
+        if constexpr (T == 1) __syncwarp();
+        else __syncthreads();
         if constexpr (DM == 3) i8_prep_query(s, v.dim);
-        uint32_t cur = v.enterpoint;
-        float curd = warp_dist_one<DM>(v, s.q, cur);
-        c_dist++;
-        greedy_descent<DM>(v, s, v.maxlevel, 0, cur, curd, c_dist);
-        c_dist++;  // the reference evaluates the entry point again (hrnn.h:505)
-        uint32_t tsize = beam_search<DM>(v, s, cur, curd, EF, 0, vc, c_dist, c_exp);
+        uint32_t cur = v.enterpoint, tsize;
+        float curd = 0.f;
+        if (T == 1 || w == 0) {
+            curd = warp_dist_one<DM, RK>(v, s.q, cur);
+            greedy_descent<DM, RK>(v, s, v.maxlevel, 0, cur, curd, c_dist);
+            c_dist += 2;  // the entry point twice, like the reference (hrnn.h:505)
+        }
+        if constexpr (T == 1) {
+            tsize = beam_search<DM, RK>(v, s, cur, curd, EF, 0, vc, c_dist, c_exp);
+        } else {
+            // (warp 0's cur and curd reach the others through the beam's first entry)
+            uint32_t* ids2 = (uint32_t*)(smem_raw + warp_smem_bytes(v.dim, efc, vc));
+            tsize = EF <= 256 ? beam_search_team<DM == 1, RK, 8>(v, s, ids2, cur, curd, EF, 0, vc, c_dist, c_exp)
+                              : beam_search_team<DM == 1, RK, 16>(v, s, ids2, cur, curd, EF, 0, vc, c_dist, c_exp);
+        }
         uint32_t np_ = min(min(max(m, m_keep), mmax), tsize);
-        for (uint32_t i = lane; i < np_; i += 32) {
+        for (uint32_t i = ut; i < np_; i += un) {
             prox[(size_t)qi * mmax + i] = s.ti[i] & kIdMask;
             if (proxd) proxd[(size_t)qi * mmax + i] = s.td[i];
         }
-        if (lane == 0) nprox[qi] = np_;
-        __syncwarp();
+        if (ut == 0) nprox[qi] = np_;
+        if constexpr (T == 1) __syncwarp();
+        else __syncthreads();
     }
     if (lane == 0) {
         atomicAdd(&ctr->n_dist, c_dist);
@@ -188,7 +210,7 @@ __global__ void __launch_bounds__(128, R2 ? 4 : 1) k_phase_a_fast(DevView v, con
             uint32_t cur = v.enterpoint;
             float curd = warp_dist_one<DM>(v, s.q, cur);
             c_dist++;
-            greedy_descent<DM>(v, s, v.maxlevel, 0, cur, curd, c_dist);
+            greedy_descent<DM, kRowsAny>(v, s, v.maxlevel, 0, cur, curd, c_dist);
             if (lane == 0) {
                 s.td[0] = curd;
                 s.ti[0] = cur;
@@ -500,6 +522,7 @@ struct PhaseA {
     bool fast;
     int dm;
     bool r2;
+    bool team;
     DevView v;
     const float* q;
     const uint32_t *qm, *qef;
@@ -508,12 +531,33 @@ struct PhaseA {
     SearchCounters* ctr;
 };
 
-static const void* phase_a_kernel(bool fast, int dm, bool r2) {
+using KPhaseA = void (*)(DevView, const float*, uint32_t, const uint32_t*, const uint32_t*, uint32_t, uint32_t, uint32_t,
+                         uint32_t*, uint32_t*, SearchCounters*, const uint32_t*, uint32_t, uint32_t, uint32_t, float*,
+                         uint32_t*, const uint32_t*);
+
+// Whether a batch gets a team of warps per query (exact forms): too few queries to
+// fill the device, and link rows and beam as beam_search_team takes them.
+static bool phase_a_team(bool fast, int dm, const DevView& v, size_t nq, uint32_t efc, int nsm) {
+    return !fast && dm < 2 && nq <= team_searches(nsm) && efc <= kTeamMaxEf && v.W0 <= 33 &&
+           rows_kind(v.dim, v.lanes) != kRowsAny && warp_smem_bytes(v.dim, efc, team_vis(efc)) + 256 <= 227 * 1024;
+}
+
+// The reference-order kernel of a distance mode and the view's rows.
+static KPhaseA phase_a_exact(int dm, const DevView& v, bool team) {
+    if (dm == 3) return k_phase_a<3, kRowsAny, 1>;
+    if (dm == 2) return k_phase_a<2, kRowsAny, 1>;
+    return with_rows(rows_kind(v.dim, v.lanes), [&](auto rk) -> KPhaseA {
+        constexpr int RK = decltype(rk)::value;
+        if constexpr (RK != kRowsAny)
+            if (team) return dm == 1 ? k_phase_a<1, RK, kTeamWarps> : k_phase_a<0, RK, kTeamWarps>;
+        return dm == 1 ? k_phase_a<1, RK, 1> : k_phase_a<0, RK, 1>;
+    });
+}
+
+static const void* phase_a_kernel(bool fast, int dm, bool r2, const DevView& v, bool team) {
     return fast ? (dm == 3 ? (r2 ? (const void*)k_phase_a_fast<3, true> : (const void*)k_phase_a_fast<3, false>)
                            : (const void*)k_phase_a_fast<2, false>)
-                : (dm == 3 ? (const void*)k_phase_a<3>
-                           : dm == 2 ? (const void*)k_phase_a<2>
-                                     : dm == 1 ? (const void*)k_phase_a<1> : (const void*)k_phase_a<0>);
+                : (const void*)phase_a_exact(dm, v, team);
 }
 
 // One launch; qlist / m_over / ef_over / m_keep / proxd / save / resume / nq_dev as
@@ -527,8 +571,7 @@ static void launch_phase_a(const PhaseA& p, unsigned g, int cw, uint32_t cv, siz
         k<<<g, cw * 32, sm, ls>>>(p.v, p.q, nqq, p.qm, p.qef, p.efc, cv, p.mmax, p.prox, p.nprox, p.ctr, qlist, m_over,
                                   ef_over, m_keep, proxd, ctrq, save_cap, st_cnt, st_d, st_i, resume, nq_dev);
     } else {
-        auto k = p.dm == 3 ? k_phase_a<3> : p.dm == 2 ? k_phase_a<2> : p.dm == 1 ? k_phase_a<1> : k_phase_a<0>;
-        k<<<g, cw * 32, sm, ls>>>(p.v, p.q, nqq, p.qm, p.qef, p.efc, cv, p.mmax, p.prox, p.nprox, p.ctr, qlist, m_over,
+        phase_a_exact(p.dm, p.v, p.team)<<<g, cw * 32, sm, ls>>>(p.v, p.q, nqq, p.qm, p.qef, p.efc, cv, p.mmax, p.prox, p.nprox, p.ctr, qlist, m_over,
                                   ef_over, m_keep, proxd, ctrq, nq_dev);
     }
     CUDA_LAUNCH_CHECK();
@@ -633,8 +676,11 @@ uint64_t search_batch(Index& ix, const SearchArgs& a) {
         const int dm = int8 ? 3 : mixed ? 2 : fusedsimd ? 1 : 0;
         // r2: the INT8 two-parent search loads all 64 rows of a step at once (a launch-shape choice)
         bool r2 = false;
-        auto kfun_of = [&](bool two) { return phase_a_kernel(fast, dm, two); };
+        const bool team = !learned && phase_a_team(fast, dm, v, nq, efc, nsm);
+        if (team) vc = team_vis(efc);
+        auto kfun_of = [&](bool two) { return phase_a_kernel(fast, dm, two, v, team); };
         auto smem_for = [&](uint32_t cv, int cw) {
+            if (team) return warp_smem_bytes(v.dim, efc, cv) + 256;  // one search, and its scored neighbours' ids
             return (fast ? fast_smem_bytes(v.dim, efc, cv) : warp_smem_bytes(v.dim, efc, cv)) * (size_t)cw;
         };
         // One launch of the form's phase-A kernel; qlist / ef_over / m_keep / proxd /
@@ -644,7 +690,7 @@ uint64_t search_batch(Index& ix, const SearchArgs& a) {
         auto launch = [&](unsigned g, int cw, uint32_t cv, size_t sm, uint32_t nqq, const uint32_t* qlist,
                           uint32_t m_over, uint32_t ef_over, uint32_t m_keep, float* proxd, uint32_t* ctrq,
                           uint32_t save_cap, uint32_t* st_cnt, float* st_d, uint32_t* st_i, int resume) {
-            PhaseA pa{fast, dm, r2, v, a.d_q, a.d_m, a.d_ef, efc, mmax, prox.as<uint32_t>(), nprox.as<uint32_t>(), ctr};
+            PhaseA pa{fast, dm, r2, team, v, a.d_q, a.d_m, a.d_ef, efc, mmax, prox.as<uint32_t>(), nprox.as<uint32_t>(), ctr};
             launch_phase_a(pa, g, cw, cv, sm, ls, nqq, qlist, m_over, ef_over, m_keep, proxd, ctrq, save_cap, st_cnt,
                            st_d, st_i, resume, nullptr);
         };
@@ -653,7 +699,9 @@ uint64_t search_batch(Index& ix, const SearchArgs& a) {
         // now on this batch when autotuning is on and the batch is large enough.
         const uint64_t shape_key = ((uint64_t)dm << 32) | efc;
         auto shape = ix.autotune ? ix.a_shape.find(shape_key) : ix.a_shape.end();
-        if (shape != ix.a_shape.end()) {
+        if (team) {
+            wpb = kTeamWarps;
+        } else if (shape != ix.a_shape.end()) {
             wpb = (int)(shape->second.first & 0xFF);
             r2 = (shape->second.first & 0x100) != 0;
             vc = shape->second.second;
@@ -712,7 +760,8 @@ uint64_t search_batch(Index& ix, const SearchArgs& a) {
         int per_sm = 1;
         CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfun, wpb * 32, smem_a));
         auto grid_for = [&](size_t n) {
-            return (unsigned)std::max<size_t>(1, std::min<size_t>((n + wpb - 1) / wpb, (size_t)nsm * std::max(per_sm, 1)));
+            const size_t blocks = team ? n : (n + wpb - 1) / wpb;
+            return (unsigned)std::max<size_t>(1, std::min<size_t>(blocks, (size_t)nsm * std::max(per_sm, 1)));
         };
         if (!learned) {
             launch(grid_for(nq), wpb, vc, smem_a, (uint32_t)nq, nullptr, 0, 0, 0, nullptr, d_qa, 0, nullptr, nullptr,
@@ -1022,7 +1071,7 @@ void budget_features(Index& ix, const float* d_q, size_t nq, uint32_t k, uint32_
                                             proxd.as<float>(), next.as<uint32_t>(), 0, nullptr, nullptr, nullptr, 0,
                                             nullptr);
     } else {
-        auto kern = int8 ? k_phase_a<3> : mixed ? k_phase_a<2> : ((ix.order.fused & 1) != 0) ? k_phase_a<1> : k_phase_a<0>;
+        auto kern = phase_a_exact(int8 ? 3 : mixed ? 2 : (ix.order.fused & 1) != 0 ? 1 : 0, v, false);
         CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
         kern<<<grid, wpb * 32, smem_a, s>>>(v, d_q, (uint32_t)nq, nullptr, nullptr, efc, vc, mmax,
                                             prox.as<uint32_t>(), nprox.as<uint32_t>(),
@@ -1059,7 +1108,7 @@ namespace {
 struct PlanLaunch {
     uint32_t efc, vc, mmax, mstride, reserve, wpb, grid_a, grid_bc, kidx, slots, hcap;
     size_t smem_a, smem_bc, smem_w, tmax;
-    bool mixed, int8, fusedsimd, counts, fast, r2, learned, two_pass;
+    bool mixed, int8, fusedsimd, counts, fast, r2, learned, two_pass, team;
 };
 
 PlanLaunch plan_launch_shape(Index& ix, const SearchPlan& p) {
@@ -1086,13 +1135,20 @@ PlanLaunch plan_launch_shape(Index& ix, const SearchPlan& p) {
     };
     L.wpb = (uint32_t)std::max<size_t>(1, std::min<size_t>(4, (200 * 1024) / wsm_of(L.vc)));
     L.smem_a = wsm_of(L.vc) * L.wpb;
-    const uint64_t shape_key = ((uint64_t)(L.int8 ? 3 : L.mixed ? 2 : L.fusedsimd ? 1 : 0) << 32) | L.efc;
+    const int dm = L.int8 ? 3 : L.mixed ? 2 : L.fusedsimd ? 1 : 0;
+    const uint64_t shape_key = ((uint64_t)dm << 32) | L.efc;
     auto shape = ix.autotune ? ix.a_shape.find(shape_key) : ix.a_shape.end();  // tuned by an earlier batch call
     if (shape != ix.a_shape.end()) {
         L.wpb = shape->second.first & 0xFF;
         L.r2 = (shape->second.first & 0x100) != 0;
         L.vc = shape->second.second;
         L.smem_a = wsm_of(L.vc) * L.wpb;
+    }
+    L.team = !L.learned && phase_a_team(L.fast, dm, v, p.nq, L.efc, sms(ix.device));
+    if (L.team) {
+        L.wpb = kTeamWarps;
+        L.vc = team_vis(L.efc);
+        L.smem_a = wsm_of(L.vc) + 256;
     }
     L.counts = p.threshold > 1.0f;
     L.kidx = p.k - 1;
@@ -1250,11 +1306,11 @@ void plan_create(SearchPlan& p, cudaStream_t s) {
     exclusive_scan_u64(d_total, d_resoff, nq + 1, s, p.tmp);
     exclusive_scan_u32_to_u64(d_rcount, p.d_out_off, nq + 1, s, p.tmp);
     const int dm = L.int8 ? 3 : L.mixed ? 2 : L.fusedsimd ? 1 : 0;
-    const void* kfun = phase_a_kernel(L.fast, dm, L.r2);
+    const void* kfun = phase_a_kernel(L.fast, dm, L.r2, v, L.team);
     CUDA_CHECK(cudaFuncSetAttribute(kfun, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem_a));
     int per_sm = 1;
     CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfun, L.wpb * 32, L.smem_a));
-    L.grid_a = (uint32_t)std::max<size_t>(1, std::min<size_t>((nq + L.wpb - 1) / L.wpb, (size_t)nsm * std::max(per_sm, 1)));
+    L.grid_a = (uint32_t)std::max<size_t>(1, std::min<size_t>(L.team ? nq : (nq + L.wpb - 1) / L.wpb, (size_t)nsm * std::max(per_sm, 1)));
     KCta kc = ix.wide ? pick_bc<uint64_t>(L.fusedsimd, L.counts, L.mixed) : pick_bc<uint32_t>(L.fusedsimd, L.counts, L.mixed);
     if (stream) {
         p.sb.reserve((uint32_t)nq, v.dim, nq * L.mstride, stream_max_chunks(nq * L.tmax, nq * L.mstride));
@@ -1286,7 +1342,7 @@ void plan_create(SearchPlan& p, cudaStream_t s) {
                                                                flag);
     // the per-call column of kdist(p, k-1) (hrnn.h:286-293): features and verification
     k_kdist_column<<<(unsigned)((ix.cur + 255) / 256), 256, 0, s>>>(v, L.kidx, p.kcol.as<float>());
-    const PhaseA pa{L.fast, dm, L.r2, v, p.d_q, pm, pef, L.efc, L.mstride, p.prox.as<uint32_t>(),
+    const PhaseA pa{L.fast, dm, L.r2, L.team, v, p.d_q, pm, pef, L.efc, L.mstride, p.prox.as<uint32_t>(),
                     p.nprox.as<uint32_t>(), ctr};
     if (!bud) {
         launch_phase_a(pa, L.grid_a, (int)L.wpb, L.vc, L.smem_a, s, (uint32_t)nq, nullptr, 0, 0, 0, nullptr, d_next + 4,
