@@ -978,14 +978,17 @@ struct QuadRow<FUSED, kRows4> {
     }
 };
 
+__device__ __forceinline__ void touch(const uint32_t* p) {
+    asm volatile("{\n .reg .u32 w;\n ld.global.nc.u32 w, [%0];\n}" ::"l"(p));
+}
+
 // The level-0 link row of `node`, towards L1: the quad's lanes read one word of each
 // of its 32-byte sectors.
 __device__ __forceinline__ void quad_touch_links(const DevView& v, uint32_t node) {
     const uint32_t* row = v.adj0 + (size_t)node * v.W0;
     const uint32_t at = 8 * (threadIdx.x & 3);
-    uint32_t sink;
-    if (at < v.W0) asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(sink) : "l"(row + at));
-    if (at == 0) asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(sink) : "l"(row + v.W0 - 1));
+    if (at < v.W0) touch(row + at);
+    if (at == 0) touch(row + v.W0 - 1);
 }
 
 // beam_search by a block of kTeamWarps warps (link rows of at most 33 words, EF <= 32

@@ -19,6 +19,7 @@
 #include <cfloat>
 #include <vector>
 
+#include "csr_kernels.cuh"
 #include "index.hpp"
 
 namespace hrnn {
@@ -36,21 +37,11 @@ __global__ void k_degree(const uint32_t* __restrict__ ids, const uint32_t* __res
     }
 }
 
-template <class E>
-__global__ void k_scatter(const uint32_t* __restrict__ ids, const uint32_t* __restrict__ hdr, size_t n,
-                          uint32_t K, const uint64_t* __restrict__ off, uint32_t* __restrict__ cursor,
-                          E* __restrict__ ent, uint32_t rb) {
-    size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    size_t nw = ((size_t)gridDim.x * blockDim.x) >> 5;
-    for (size_t i = warp; i < n; i += nw) {
-        uint32_t c = hdr[i] & 0xFFFFu;
-        for (uint32_t j = lane; j < c; j += 32) {
-            uint32_t nbr = ids[i * K + j];
-            uint64_t pos = off[nbr] + atomicAdd(&cursor[nbr], 1u);
-            ent[pos] = (E)(((uint64_t)i << rb) | j);
-        }
-    }
+// The scatter's cursors: every segment's first place.
+template <class C>
+__global__ void k_cursors(const uint64_t* __restrict__ off, size_t n, C* __restrict__ cursor) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) cursor[i] = (C)off[i];
 }
 
 // Sort key: rank in the high word, owner in the low word.
@@ -63,9 +54,6 @@ template <class E>
 __device__ __forceinline__ E from_key(uint64_t k, uint32_t rb) {
     return (E)(((k & 0xFFFFFFFFull) << rb) | (k >> 32));
 }
-
-constexpr int kWarpSegMax = 1024;
-constexpr int kSortWarps = 4;
 
 // Bitonic sort of P (power of two) keys in shared memory by a group of `nthreads`
 // threads with thread index t; sync() separates the stages.
@@ -86,32 +74,6 @@ __device__ void bitonic(uint64_t* s, uint32_t P, uint32_t t, uint32_t nthreads, 
             }
             sync();
         }
-    }
-}
-
-template <class E>
-__global__ void k_sort_small(const uint64_t* __restrict__ off, size_t n, E* __restrict__ ent, uint32_t rb,
-                             uint32_t* __restrict__ big, uint32_t* __restrict__ n_big) {
-    __shared__ uint64_t sm[kSortWarps][kWarpSegMax];
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    size_t seg = (size_t)blockIdx.x * kSortWarps + w;
-    size_t stride = (size_t)gridDim.x * kSortWarps;
-    for (; seg < n; seg += stride) {
-        uint64_t b = off[seg], e = off[seg + 1];
-        uint32_t len = (uint32_t)(e - b);
-        if (len <= 1) continue;
-        if (len > kWarpSegMax) {
-            if (lane == 0) big[atomicAdd(n_big, 1u)] = (uint32_t)seg;
-            continue;
-        }
-        uint32_t P = 32;
-        while (P < len) P <<= 1;
-        uint64_t* s = sm[w];
-        for (uint32_t i = lane; i < P; i += 32) s[i] = i < len ? to_key<E>(ent[b + i], rb) : ~0ull;
-        __syncwarp();
-        bitonic(s, P, lane, 32, [] { __syncwarp(); });
-        for (uint32_t i = lane; i < len; i += 32) ent[b + i] = from_key<E>(s[i], rb);
-        __syncwarp();
     }
 }
 
@@ -159,9 +121,8 @@ void build_impl(Index& ix) {
     DevMem& big = ix.scratch[2];
     DevMem& tmp = ix.scratch[3];
     deg.ensure((n + 1) * 4);
-    cursor.ensure((n + 1) * 4 + 4);
+    cursor.ensure((n + 2) * 8);
     CUDA_CHECK(cudaMemsetAsync(deg.p, 0, (n + 1) * 4, s));
-    CUDA_CHECK(cudaMemsetAsync(cursor.p, 0, (n + 1) * 4 + 4, s));
     int grid = sm_count(ix.device) * 8;
     k_degree<<<grid, 256, 0, s>>>(ix.knn_ids.as<uint32_t>(), ix.knn_hdr.as<uint32_t>(), n, (uint32_t)K,
                                   deg.as<uint32_t>());
@@ -172,30 +133,28 @@ void build_impl(Index& ix) {
     CUDA_CHECK(cudaMemcpyAsync(&total, ix.csr_off.as<uint64_t>() + n, 8, cudaMemcpyDeviceToHost, s));
     CUDA_CHECK(cudaStreamSynchronize(s));
     ix.csr_ent.ensure(std::max<uint64_t>(total, 1) * sizeof(E));
-    k_scatter<E><<<grid, 256, 0, s>>>(ix.knn_ids.as<uint32_t>(), ix.knn_hdr.as<uint32_t>(), n, (uint32_t)K,
-                                      ix.csr_off.as<uint64_t>(), cursor.as<uint32_t>(), ix.csr_ent.as<E>(),
-                                      ix.rank_bits);
-    CUDA_LAUNCH_CHECK();
+    auto scatter = [&](auto c) {
+        using C = decltype(c);
+        k_cursors<C><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(ix.csr_off.as<uint64_t>(), n, cursor.as<C>());
+        CUDA_LAUNCH_CHECK();
+        k_scatter_edges<E, C><<<grid, 256, 0, s>>>(ix.knn_ids.as<uint32_t>(), ix.knn_hdr.as<uint32_t>(), n,
+                                                   (uint32_t)K, cursor.as<C>(), ix.csr_ent.as<E>(), ix.rank_bits, Guard{});
+        CUDA_LAUNCH_CHECK();
+    };
+    if (total >> 32) scatter((unsigned long long)0);
+    else scatter(0u);
     big.ensure((n + 1) * 4);
-    uint32_t* n_big = cursor.as<uint32_t>() + n + 1;  // spare word, zeroed above
-    CUDA_CHECK(cudaMemsetAsync(n_big, 0, 4, s));
-    size_t blocks = std::min<size_t>((n + kSortWarps - 1) / kSortWarps, (size_t)sm_count(ix.device) * 32);
-    k_sort_small<E><<<(unsigned)std::max<size_t>(blocks, 1), kSortWarps * 32, 0, s>>>(
-        ix.csr_off.as<uint64_t>(), n, ix.csr_ent.as<E>(), ix.rank_bits, big.as<uint32_t>(), n_big);
+    uint32_t* n_big = (uint32_t*)(cursor.as<uint64_t>() + n + 1);  // beyond the cursors: listed segments, largest
+    CUDA_CHECK(cudaMemsetAsync(n_big, 0, 8, s));
+    size_t blocks = std::min<size_t>((n + kSegWarps - 1) / kSegWarps, (size_t)sm_count(ix.device) * 32);
+    k_sort_segments<E><<<(unsigned)std::max<size_t>(blocks, 1), kSegWarps * 32, 0, s>>>(
+        ix.csr_off.as<uint64_t>(), n, ix.csr_ent.as<E>(), ix.rank_bits, big.as<uint32_t>(), n_big, n_big + 1, Guard{});
     CUDA_LAUNCH_CHECK();
-    uint32_t nb = 0;
-    CUDA_CHECK(cudaMemcpyAsync(&nb, n_big, 4, cudaMemcpyDeviceToHost, s));
+    uint32_t nbp[2] = {0, 0};
+    CUDA_CHECK(cudaMemcpyAsync(nbp, n_big, 8, cudaMemcpyDeviceToHost, s));
     CUDA_CHECK(cudaStreamSynchronize(s));
+    const uint32_t nb = nbp[0], P = nbp[1];
     if (nb) {
-        // Size the staging area for the largest segment.
-        std::vector<uint32_t> bigs(nb);
-        CUDA_CHECK(cudaMemcpy(bigs.data(), big.p, nb * 4, cudaMemcpyDeviceToHost));
-        std::vector<uint64_t> hoff(n + 1);
-        CUDA_CHECK(cudaMemcpy(hoff.data(), ix.csr_off.p, (n + 1) * 8, cudaMemcpyDeviceToHost));
-        uint32_t maxlen = 0;
-        for (uint32_t sg : bigs) maxlen = std::max<uint32_t>(maxlen, (uint32_t)(hoff[sg + 1] - hoff[sg]));
-        uint32_t P = 32;
-        while (P < maxlen) P <<= 1;
         const uint32_t smem_keys = 16384;  // 128 KB
         uint64_t* gtmp = nullptr;
         size_t stride = 0;

@@ -25,6 +25,7 @@
 #include <mutex>
 #include <string>
 
+#include "csr_kernels.cuh"
 #include "index.hpp"
 
 namespace hrnn {
@@ -32,7 +33,6 @@ namespace {
 
 constexpr size_t kScratchBytes = 32ull << 20;  // 32 MiB, held by every device that loads the library
 constexpr size_t kMaxN = 1ull << 21;           // 2,097,152 elements
-constexpr int kNaWarpSegMax = 1024;
 constexpr int kNaSmemKeys = 16384;
 constexpr int kScanT = 512, kScanPer = 8, kScanTile = kScanT * kScanPer;
 
@@ -96,10 +96,16 @@ __global__ void na_degree(const uint32_t* __restrict__ ids, const uint32_t* __re
             if (lane == 0) atomicAdd(&bad[0], 1u);
             continue;
         }
-        for (uint32_t j = lane; j < c; j += 32) {
-            const uint32_t id = ids[i * K + j];
-            if (id < n) atomicAdd(&deg[id], 1u);
-            else atomicAdd(&bad[1], 1u);
+        for (uint32_t j0 = lane; j0 < c; j0 += 32 * kEdgeU) {
+            uint32_t id[kEdgeU];
+#pragma unroll
+            for (int u = 0; u < kEdgeU; ++u) id[u] = j0 + 32 * u < c ? ids[i * K + j0 + 32 * u] : 0u;
+#pragma unroll
+            for (int u = 0; u < kEdgeU; ++u)
+                if (j0 + 32 * u < c) {
+                    if (id[u] < n) atomicAdd(&deg[id[u]], 1u);
+                    else atomicAdd(&bad[1], 1u);
+                }
         }
     }
 }
@@ -155,26 +161,18 @@ __global__ void na_scan_parts(uint64_t* part, size_t tiles) {
     }
 }
 
-__global__ void na_scan_add(uint64_t* __restrict__ out, size_t n, const uint64_t* __restrict__ part) {
-    size_t base = (size_t)blockIdx.x * kScanTile;
+// Adds the tiles' bases, and starts the scatter's cursors there.
+template <class C>
+__global__ void na_scan_add(uint64_t* __restrict__ out, size_t n, const uint64_t* __restrict__ part,
+                            C* __restrict__ cursor) {
+    const size_t base = (size_t)blockIdx.x * kScanTile;
+    const uint64_t add = part[blockIdx.x];
     for (int k = threadIdx.x; k < kScanTile; k += kScanT)
-        if (base + k < n) out[base + k] += part[blockIdx.x];
-}
-
-template <class E>
-__global__ void na_scatter(const uint32_t* __restrict__ ids, const uint32_t* __restrict__ cnt, size_t n, uint32_t K,
-                           const uint64_t* __restrict__ off, uint32_t* __restrict__ cursor, E* __restrict__ ent,
-                           uint32_t rb) {
-    size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    size_t nw = ((size_t)gridDim.x * blockDim.x) >> 5;
-    for (size_t i = warp; i < n; i += nw) {
-        uint32_t c = cnt[i] & 0xFFFFu;
-        for (uint32_t j = lane; j < c; j += 32) {
-            uint32_t nbr = ids[i * K + j];
-            ent[off[nbr] + atomicAdd(&cursor[nbr], 1u)] = (E)(((uint64_t)i << rb) | j);
+        if (base + k < n) {
+            const uint64_t o = out[base + k] + add;
+            out[base + k] = o;
+            cursor[base + k] = (C)o;
         }
-    }
 }
 
 template <class E>
@@ -205,35 +203,6 @@ __device__ void na_bitonic(uint64_t* s, uint32_t P, uint32_t t, uint32_t nt, Syn
         }
 }
 
-// Segments up to 1024 entries, one warp each; longer ones are listed in `big`
-// and their largest power-of-two size is tracked in *maxP.
-template <class E>
-__global__ void na_sort_small(const uint64_t* __restrict__ off, size_t n, E* __restrict__ ent, uint32_t rb,
-                              uint32_t* __restrict__ big, uint32_t* __restrict__ nbig, uint32_t* __restrict__ maxP) {
-    __shared__ uint64_t sm[4][kNaWarpSegMax];
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (size_t seg = (size_t)blockIdx.x * 4 + w; seg < n; seg += (size_t)gridDim.x * 4) {
-        uint64_t b = off[seg];
-        uint32_t len = (uint32_t)(off[seg + 1] - b);
-        if (len <= 1) continue;
-        uint32_t P = 32;
-        while (P < len) P <<= 1;
-        if (len > kNaWarpSegMax) {
-            if (lane == 0) {
-                big[atomicAdd(nbig, 1u)] = (uint32_t)seg;
-                atomicMax(maxP, P);
-            }
-            continue;
-        }
-        uint64_t* s = sm[w];
-        for (uint32_t i = lane; i < P; i += 32) s[i] = i < len ? na_key<E>(ent[b + i], rb) : ~0ull;
-        __syncwarp();
-        na_bitonic(s, P, lane, 32, [] { __syncwarp(); });
-        for (uint32_t i = lane; i < len; i += 32) ent[b + i] = na_entry<E>(s[i], rb);
-        __syncwarp();
-    }
-}
-
 // One block per long segment; keys in dynamic shared memory when they fit,
 // otherwise in the staging area (stride words per block).
 template <class E>
@@ -259,17 +228,20 @@ uint64_t transpose(const uint32_t* ids, const uint32_t* cnt, size_t n, uint32_t 
                    void* entries, size_t cap, char* base, cudaStream_t s, int nsm) {
     // scratch layout
     const size_t tiles = (n + 1 + kScanTile - 1) / kScanTile;
+    // (cursors of 8 bytes where n K edges may pass 2^32 take the list's place too, and
+    // the list that of the counters, which the prefix sum was the last to read)
+    const bool wide_cursor = (uint64_t)n * K >> 32;
+    const size_t words = al256((n + 1) * 4);
     uint32_t* deg = (uint32_t*)base;
-    uint32_t* cursor = (uint32_t*)(base + al256((n + 1) * 4));
-    uint32_t* big = (uint32_t*)((char*)cursor + al256((n + 1) * 4));
-    uint64_t* part = (uint64_t*)((char*)big + al256((n + 1) * 4));
+    char* cursor = base + words;
+    uint32_t* big = wide_cursor ? deg : (uint32_t*)(cursor + words);
+    uint64_t* part = (uint64_t*)(cursor + 2 * words);
     // ctl: [0] n_big, [1] max P, [2] counts above K, [3] ids >= n
     uint32_t* ctl = (uint32_t*)((char*)part + al256(tiles * 8));
     uint64_t* stage = (uint64_t*)((char*)ctl + 256);
     const size_t used = (size_t)((char*)stage - base);
     const size_t stage_words = (kScratchBytes - used) / 8;
     CUDA_CHECK(cudaMemsetAsync(deg, 0, (n + 1) * 4, s));
-    CUDA_CHECK(cudaMemsetAsync(cursor, 0, (n + 1) * 4, s));
     CUDA_CHECK(cudaMemsetAsync(ctl, 0, 16, s));
     const int grid = nsm * 8;
     na_degree<<<grid, 256, 0, s>>>(ids, cnt, n, K, deg, ctl + 2);
@@ -278,26 +250,32 @@ uint64_t transpose(const uint32_t* ids, const uint32_t* cnt, size_t n, uint32_t 
     CUDA_LAUNCH_CHECK();
     na_scan_parts<<<1, 32, 0, s>>>(part, tiles);
     CUDA_LAUNCH_CHECK();
-    na_scan_add<<<(unsigned)tiles, kScanT, 0, s>>>(off, n + 1, part);
+    if (wide_cursor)
+        na_scan_add<<<(unsigned)tiles, kScanT, 0, s>>>(off, n + 1, part, (unsigned long long*)cursor);
+    else
+        na_scan_add<<<(unsigned)tiles, kScanT, 0, s>>>(off, n + 1, part, (uint32_t*)cursor);
+    CUDA_LAUNCH_CHECK();
+    // the checks of the graph and of the entries' capacity are made on the device too
+    // (Guard), so one wait covers the whole transpose
+    const Guard guard{off + n, cap, ctl + 2};
+    E* ent = static_cast<E*>(entries);
+    if (wide_cursor)
+        k_scatter_edges<E><<<grid, 256, 0, s>>>(ids, cnt, n, K, (unsigned long long*)cursor, ent, rb, guard);
+    else
+        k_scatter_edges<E><<<grid, 256, 0, s>>>(ids, cnt, n, K, (uint32_t*)cursor, ent, rb, guard);
+    CUDA_LAUNCH_CHECK();
+    const unsigned blocks = (unsigned)std::min<size_t>((n + kSegWarps - 1) / kSegWarps, (size_t)nsm * 32);
+    k_sort_segments<E><<<blocks ? blocks : 1, 32 * kSegWarps, 0, s>>>(off, n, ent, rb, big, ctl, ctl + 1, guard);
     CUDA_LAUNCH_CHECK();
     uint64_t total = 0;
-    uint32_t badc[2] = {0, 0};
+    uint32_t hc[4] = {0, 0, 0, 0};
     CUDA_CHECK(cudaMemcpyAsync(&total, off + n, 8, cudaMemcpyDeviceToHost, s));
-    CUDA_CHECK(cudaMemcpyAsync(badc, ctl + 2, 8, cudaMemcpyDeviceToHost, s));
+    CUDA_CHECK(cudaMemcpyAsync(hc, ctl, 16, cudaMemcpyDeviceToHost, s));
     CUDA_CHECK(cudaStreamSynchronize(s));
-    if (badc[0] || badc[1])
-        fail(HRNN_ERR_ARG, "build_rknng_noalloc: the graph has " + std::to_string(badc[0]) +
-                               " count(s) above K and " + std::to_string(badc[1]) + " neighbour id(s) >= n");
+    if (hc[2] || hc[3])
+        fail(HRNN_ERR_ARG, "build_rknng_noalloc: the graph has " + std::to_string(hc[2]) +
+                               " count(s) above K and " + std::to_string(hc[3]) + " neighbour id(s) >= n");
     if (total > cap) return total;  // caller's entry buffer too small: report the need
-    E* ent = static_cast<E*>(entries);
-    na_scatter<E><<<grid, 256, 0, s>>>(ids, cnt, n, K, off, cursor, ent, rb);
-    CUDA_LAUNCH_CHECK();
-    unsigned blocks = (unsigned)std::min<size_t>((n + 3) / 4, (size_t)nsm * 32);
-    na_sort_small<E><<<blocks ? blocks : 1, 128, 0, s>>>(off, n, ent, rb, big, ctl, ctl + 1);
-    CUDA_LAUNCH_CHECK();
-    uint32_t hc[2] = {0, 0};
-    CUDA_CHECK(cudaMemcpyAsync(hc, ctl, 8, cudaMemcpyDeviceToHost, s));
-    CUDA_CHECK(cudaStreamSynchronize(s));
     if (hc[0]) {
         const uint32_t P = hc[1];
         const size_t stride = P > (uint32_t)kNaSmemKeys ? P : 0;
@@ -312,8 +290,8 @@ uint64_t transpose(const uint32_t* ids, const uint32_t* cnt, size_t n, uint32_t 
             na_sort_big<E><<<cnt_b, 512, smem, s>>>(off, big, first, ent, rb, stage, stride);
             CUDA_LAUNCH_CHECK();
         }
+        CUDA_CHECK(cudaStreamSynchronize(s));
     }
-    CUDA_CHECK(cudaStreamSynchronize(s));
     return total;
 }
 
