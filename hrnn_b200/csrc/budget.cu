@@ -176,26 +176,31 @@ void budget_predict(Index& ix, const float* feat, size_t n, float* logits) {
     }
 }
 
+constexpr size_t kKeepIo = 64ull << 20;
+
 float budget_gradients(Index& ix, const float* feat, const uint8_t* labels, size_t n, float* grads) {
     Budget& b = budget_of(ix);
     if (!b.mlp.ready) fail(HRNN_ERR_STATE, "budget: the model has no weights");
     if (n == 0 || n > (1u << 20)) fail(HRNN_ERR_ARG, "budget_gradients: n must be in [1, 2^20]");
     cudaStream_t s = ix.stream;
-    DevMem X, Y, L;
-    upload(X, feat, n * kMlpIn * 4, s);
-    upload(Y, labels, n * 2, s);
-    L.alloc(4);
-    CUDA_CHECK(cudaMemsetAsync(L.p, 0, 4, s));
-    b.mlp.forward(X.as<float>(), (int)n, s);
-    b.mlp.backward(X.as<float>(), Y.as<uint8_t>(), (int)n, L.as<float>(), s);
-    size_t off = 0;
-    for (int i = 0; i < 6; ++i) {
-        CUDA_CHECK(cudaMemcpyAsync(grads + off, b.mlp.gr[i].p, b.mlp.n[i] * 4, cudaMemcpyDeviceToHost, s));
-        off += b.mlp.n[i];
-    }
+    // features | labels | loss, in a buffer kept with the budget up to kKeepIo bytes
+    const size_t xb = n * kMlpIn * 4, yb = (n * 2 + 15) & ~(size_t)15;
+    DevMem own;
+    DevMem& io = xb + yb + 16 <= kKeepIo ? b.io : own;
+    io.ensure(xb + yb + 16);
+    float* X = io.as<float>();
+    uint8_t* Y = (uint8_t*)(io.as<char>() + xb);
+    float* L = (float*)(io.as<char>() + xb + yb);
+    CUDA_CHECK(cudaMemcpyAsync(X, feat, xb, cudaMemcpyHostToDevice, s));
+    CUDA_CHECK(cudaMemcpyAsync(Y, labels, n * 2, cudaMemcpyHostToDevice, s));
+    CUDA_CHECK(cudaMemsetAsync(L, 0, 4, s));
+    b.mlp.forward(X, (int)n, s);
+    b.mlp.backward(X, Y, (int)n, L, s);
+    const size_t off = b.mlp.grad_floats();
+    CUDA_CHECK(cudaMemcpyAsync(grads, b.mlp.gr.p, off * 4, cudaMemcpyDeviceToHost, s));
     std::fill(grads + off, grads + off + 2 * kMlpIn, 0.f);
     float loss = 0.f;
-    CUDA_CHECK(cudaMemcpyAsync(&loss, L.p, 4, cudaMemcpyDeviceToHost, s));
+    CUDA_CHECK(cudaMemcpyAsync(&loss, L, 4, cudaMemcpyDeviceToHost, s));
     CUDA_CHECK(cudaStreamSynchronize(s));
     b.mlp.check_tc();
     return loss;

@@ -12,11 +12,20 @@ constexpr int kFrontier = 32;  // beam entries the features read
 
 struct Mlp {
     // parameters: W1 [H x In], b1, W2 [H x H], b2, W3 [Out x H], b3 (FP32 masters)
-    DevMem p[6], gr[6], m1[6], m2[6];
+    DevMem p[6], m1[6], m2[6];
+    DevMem gr;  // the six gradients, one after the other
     size_t n[6];
     DevMem norm;  // input normalisation: mean[In], 1/std[In] (x -> (x - mean) * inv)
     DevMem tc_err;  // set by the tensor-core layers when a bounded wait runs out
-    DevMem xn, z1, a1, z2, a2, z3, g1, g2, g3;  // normalised input, activations / gradients of one batch
+    // normalised input, activations / gradients of one batch and partial weight
+    // gradients of its row ranges, parts of one allocation
+    struct Part {
+        float* p = nullptr;
+        template <class T>
+        T* as() const { return reinterpret_cast<T*>(p); }
+    };
+    DevMem work;
+    Part xn, z1, a1, z2, a2, z3, g1, g2, g3, part, part3;
     int cap = 0;
     long step = 0;
     bool ready = false;
@@ -24,6 +33,12 @@ struct Mlp {
     Mlp();
     float* w(int l) const { return p[2 * l].as<float>(); }
     float* b(int l) const { return p[2 * l + 1].as<float>(); }
+    float* grad(int i) const {
+        float* g = gr.as<float>();
+        for (int j = 0; j < i; ++j) g += n[j];
+        return g;
+    }
+    size_t grad_floats() const { return n[0] + n[1] + n[2] + n[3] + n[4] + n[5]; }
     void init(uint64_t seed, cudaStream_t s);  // random weights, identity normalisation
     void ensure_work(int B);
     void forward(const float* X, int B, cudaStream_t s);  // logits in z3
@@ -47,6 +62,7 @@ struct Budget {
     DevMem proj;                  // [dim x 128] fixed random projection of the query
     uint32_t proj_dim = 0;
     DevMem feat, decided, fallback_list, proxd;  // per-call work buffers
+    DevMem io;                    // one gradient evaluation's features and labels
     DevMem saved;                 // two-pass mode: the frontier beams the fallback resumes
     unsigned long long n_level[3] = {0, 0, 0};  // queries served at level 0 / 1 / fallback (last call)
 };

@@ -4,21 +4,23 @@
 //
 // with both operands rounded to BF16 as they are staged into shared memory (the
 // same rounding as the CUDA-core GEMM of mlp.cu) and the products accumulated in
-// FP32 in tensor memory.  One CTA of 128 threads per 128-row tile:
+// FP32 in tensor memory.  One CTA of 512 threads per 128 x 64 output tile: at 4096 rows
+// that is 128 CTAs, and a layer is bound by staging and by the GELU epilogue, not by
+// the products (44 us with 128 threads on 128 x 256 tiles, 30 with 512 threads).
 //
-//   1. warp 0 allocates 256 TMEM columns (a 128 x 256 FP32 accumulator);
-//   2. all threads stage A's tile (128 x 256) and W (256 x 256) as BF16 in the
+//   1. warp 0 allocates 64 TMEM columns (a 128 x 64 FP32 accumulator);
+//   2. all threads stage A's tile (128 x 256) and 64 rows of W (64 x 256) as BF16 in the
 //      canonical K-major, no-swizzle layout: 8-row x 16-byte core matrices, the
 //      16 core matrices of a 128-byte K slab adjacent (leading byte offset 128),
 //      8-row groups 4096 bytes apart (stride byte offset);
-//   3. one thread issues the 16 tcgen05.mma (M=128, N=256, K=16 each) and
+//   3. one thread issues the 16 tcgen05.mma (M=128, N=64, K=16 each) and
 //      commits them to an mbarrier; every thread waits on it (bounded);
-//   4. warp w reads TMEM lanes 32w..32w+31 (its 32 rows) 16 columns at a time
-//      with tcgen05.ld, adds the bias, applies GELU and writes the outputs;
+//   4. warp w reads TMEM lanes 32 (w mod 4) .. + 31 (its 32 rows), a quarter of the
+//      columns per group of four warps, 16 at a time with tcgen05.ld, adds the bias, applies GELU and writes the outputs;
 //   5. warp 0 frees the TMEM columns.
 //
-// Shared memory 192 KB: one CTA per SM, so the allocation never waits on
-// another CTA's columns.
+// Shared memory 96 KB: two CTAs per SM at most, with room for both's columns, so the
+// allocation never waits on another CTA's.
 #include <cuda_bf16.h>
 
 #include <cstdint>
@@ -30,11 +32,12 @@ namespace hrnn {
 
 namespace {
 
-constexpr int kTM = 128, kTN = 256, kTK = 256;
+constexpr int kTM = 128, kTN = 64, kTK = 256;  // a CTA's tile; the layer has 256 columns
 constexpr uint32_t kSBO = (kTK / 8) * 128;  // bytes between 8-row core-matrix groups
 constexpr uint32_t kLBO = 128;              // bytes between K-adjacent core matrices
 constexpr size_t kSmemA = (size_t)kTM * kTK * 2, kSmemB = (size_t)kTN * kTK * 2;
 constexpr size_t kSmemTC = kSmemA + kSmemB + 64;
+constexpr int kTcThreads = 512;
 constexpr uint32_t kWaitLimit = 1u << 26;   // mbarrier polls before giving up
 
 // K-major, no-swizzle shared-memory matrix descriptor (tcgen05 "matrix
@@ -45,7 +48,7 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
 }
 
 // Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both
-// K-major, N = 256, M = 128.
+// K-major, N = 64, M = 128.
 constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTN >> 3) << 17) |
                             ((uint32_t)(kTM >> 4) << 24);
 
@@ -67,7 +70,8 @@ __device__ __forceinline__ float gelu_f(float x) { return 0.5f * x * (1.f + erff
 __device__ __forceinline__ void stage(char* smem, const float* __restrict__ src, int r0, int R, int rows,
                                       const float* __restrict__ nrm) {
     // thread -> (row, 8-element chunk): 32 chunks per row
-    for (int i = threadIdx.x; i < R * (kTK / 8); i += blockDim.x) {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < R * (kTK / 8); i += kTcThreads) {
         const int r = i >> 5, c = i & 31;
         const int gr = r0 + r;
         float v[8];
@@ -92,7 +96,7 @@ __device__ __forceinline__ void stage(char* smem, const float* __restrict__ src,
     }
 }
 
-__global__ void __launch_bounds__(128, 1) k_mlp_layer_tc(const float* __restrict__ A, int M,
+__global__ void __launch_bounds__(kTcThreads) k_mlp_layer_tc(const float* __restrict__ A, int M,
                                                          const float* __restrict__ W,
                                                          const float* __restrict__ bias,
                                                          const float* __restrict__ nrm, float* __restrict__ z_out,
@@ -104,7 +108,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_layer_tc(const float* __restrict
     uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + kSmemA + kSmemB);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + kSmemA + kSmemB + 16);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int r0 = blockIdx.x * kTM;
+    const int r0 = blockIdx.x * kTM, n0 = blockIdx.y * kTN;
 
     const uint32_t mbar_a = (uint32_t)__cvta_generic_to_shared(mbar);
     if (warp == 0) {
@@ -114,7 +118,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_layer_tc(const float* __restrict
     }
     if (tid == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar_a));
     stage(sA, A, r0, kTM, M, nrm);
-    stage(sB, W, 0, kTN, kTN, nullptr);
+    stage(sB, W, n0, kTN, kMlpH, nullptr);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic stores -> tensor-core reads
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -148,11 +152,13 @@ __global__ void __launch_bounds__(128, 1) k_mlp_layer_tc(const float* __restrict
     if (!done) {
         if (lane == 0) atomicExch(err, 1);
     } else {
-        const int row = r0 + warp * 32 + lane;
+        const int quad = warp & 3;  // the TMEM lanes this warp may read
+        const int row = r0 + quad * 32 + lane;
+        const int cpw = kTN / (kTcThreads / 128), cb = (warp >> 2) * cpw;
 #pragma unroll 1
-        for (int c0 = 0; c0 < kTN; c0 += 16) {
+        for (int c0 = cb; c0 < cb + cpw; c0 += 16) {
             uint32_t v[16];
-            const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
+            const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0;
             asm volatile(
                 "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
@@ -163,14 +169,14 @@ __global__ void __launch_bounds__(128, 1) k_mlp_layer_tc(const float* __restrict
             if (row < M) {
                 float z[16];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) z[j] = __uint_as_float(v[j]) + bias[c0 + j];
+                for (int j = 0; j < 16; ++j) z[j] = __uint_as_float(v[j]) + bias[n0 + c0 + j];
                 if (z_out) {
-                    float4* o = reinterpret_cast<float4*>(z_out + (size_t)row * kTN + c0);
+                    float4* o = reinterpret_cast<float4*>(z_out + (size_t)row * kMlpH + n0 + c0);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) o[j] = make_float4(z[4 * j], z[4 * j + 1], z[4 * j + 2], z[4 * j + 3]);
                 }
                 if (a_out) {
-                    float4* o = reinterpret_cast<float4*>(a_out + (size_t)row * kTN + c0);
+                    float4* o = reinterpret_cast<float4*>(a_out + (size_t)row * kMlpH + n0 + c0);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         float4 t = make_float4(z[4 * j], z[4 * j + 1], z[4 * j + 2], z[4 * j + 3]);
@@ -201,7 +207,7 @@ void mlp_layer_tc(const float* A, int M, const float* W, const float* bias, cons
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     CUDA_CHECK(cudaStreamIsCapturing(s, &cs));
     if (cs == cudaStreamCaptureStatusNone) mlp_layer_tc_prepare();
-    k_mlp_layer_tc<<<(unsigned)((M + kTM - 1) / kTM), 128, kSmemTC, s>>>(A, M, W, bias, nrm, out_z, out_a,
+    k_mlp_layer_tc<<<dim3((M + kTM - 1) / kTM, kMlpH / kTN), kTcThreads, kSmemTC, s>>>(A, M, W, bias, nrm, out_z, out_a,
                                                                           gelu ? 1 : 0, err);
     CUDA_LAUNCH_CHECK();
 }
