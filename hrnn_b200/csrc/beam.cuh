@@ -348,8 +348,8 @@ struct WarpSmem {
 };
 
 __host__ __device__ inline size_t warp_smem_bytes(uint32_t dim, uint32_t efc, uint32_t vc) {
-    // multiple of 16 for dim % 4 == 0 and efc % 32 == 0 (q is read as float4)
-    return (size_t)dim * 4 + (((size_t)dim + 15) & ~(size_t)15) + 16 + (size_t)(efc + 32) * 8 + (size_t)vc * 4 +
+    // a multiple of 16 (efc is one of 32), like every part's place
+    return (((size_t)dim * 4 + 15) & ~(size_t)15) + (((size_t)dim + 15) & ~(size_t)15) + 16 + (size_t)(efc + 32) * 8 + (size_t)vc * 4 +
            32 * 12 + 16;
 }
 
@@ -357,7 +357,7 @@ __host__ __device__ inline size_t warp_smem_bytes(uint32_t dim, uint32_t efc, ui
 __device__ inline WarpSmem carve(char* base, uint32_t dim, uint32_t efc, uint32_t vc) {
     WarpSmem s;
     s.q = (float*)base;
-    base += (size_t)dim * 4;
+    base += ((size_t)dim * 4 + 15) & ~(size_t)15;
     s.q8 = (int*)base;
     base += ((size_t)dim + 15) & ~(size_t)15;
     s.qm = (float4*)base;
@@ -421,35 +421,45 @@ __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w 
 // [64p, 64p+64) of every 128-byte chunk, i.e. elements 32c + 16p .. 32c + 16p + 15
 // of chunk c; accumulation order is free (FP32, fused).
 template <int NB>
-__device__ __forceinline__ float bf16_pair(const float* __restrict__ q, const uint16_t* __restrict__ x, int p) {
-    const uint4* x4 = reinterpret_cast<const uint4*>(x);
-    constexpr int NC = NB / 2;  // 32-element chunks
-    uint4 a[2 * NC];
+struct Bf16Half {  // a lane's half of a row
+    uint4 a[NB];
+    __device__ __forceinline__ void load(const uint16_t* __restrict__ x, int p) {
+        const uint4* x4 = reinterpret_cast<const uint4*>(x);
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-        a[2 * c] = __ldg(x4 + 4 * c + 2 * p);
-        a[2 * c + 1] = __ldg(x4 + 4 * c + 2 * p + 1);
-    }
-    float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint4 w = a[2 * c + h];
-            const float* qq = q + 32 * c + 16 * p + 8 * h;
-            float t;
-            t = qq[0] - bf16_lo(w.x); s0 = fmaf(t, t, s0);
-            t = qq[1] - bf16_hi(w.x); s1 = fmaf(t, t, s1);
-            t = qq[2] - bf16_lo(w.y); s0 = fmaf(t, t, s0);
-            t = qq[3] - bf16_hi(w.y); s1 = fmaf(t, t, s1);
-            t = qq[4] - bf16_lo(w.z); s0 = fmaf(t, t, s0);
-            t = qq[5] - bf16_hi(w.z); s1 = fmaf(t, t, s1);
-            t = qq[6] - bf16_lo(w.w); s0 = fmaf(t, t, s0);
-            t = qq[7] - bf16_hi(w.w); s1 = fmaf(t, t, s1);
+        for (int c = 0; c < NB / 2; ++c) {
+            a[2 * c] = __ldg(x4 + 4 * c + 2 * p);
+            a[2 * c + 1] = __ldg(x4 + 4 * c + 2 * p + 1);
         }
     }
-    float s = s0 + s1;
-    return s + __shfl_xor_sync(0xFFFFFFFFu, s, 1);  // both lanes of the pair
+    __device__ __forceinline__ float dist(const float* __restrict__ q, int p) const {
+        float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+        for (int c = 0; c < NB / 2; ++c) {  // 32-element chunks
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint4 w = a[2 * c + h];
+                const float* qq = q + 32 * c + 16 * p + 8 * h;
+                float t;
+                t = qq[0] - bf16_lo(w.x); s0 = fmaf(t, t, s0);
+                t = qq[1] - bf16_hi(w.x); s1 = fmaf(t, t, s1);
+                t = qq[2] - bf16_lo(w.y); s0 = fmaf(t, t, s0);
+                t = qq[3] - bf16_hi(w.y); s1 = fmaf(t, t, s1);
+                t = qq[4] - bf16_lo(w.z); s0 = fmaf(t, t, s0);
+                t = qq[5] - bf16_hi(w.z); s1 = fmaf(t, t, s1);
+                t = qq[6] - bf16_lo(w.w); s0 = fmaf(t, t, s0);
+                t = qq[7] - bf16_hi(w.w); s1 = fmaf(t, t, s1);
+            }
+        }
+        const float s = s0 + s1;
+        return s + __shfl_xor_sync(0xFFFFFFFFu, s, 1);  // both lanes of the pair
+    }
+};
+
+template <int NB>
+__device__ __forceinline__ float bf16_pair(const float* __restrict__ q, const uint16_t* __restrict__ x, int p) {
+    Bf16Half<NB> h;
+    h.load(x, p);
+    return h.dist(q, p);
 }
 
 // Any dim (one lane per row, scalar), for dims not a multiple of 32.
@@ -604,15 +614,26 @@ __device__ __forceinline__ float i8_one(const DevView& v, const float* q, uint32
     }
 }
 
-template <int NB>
+// G: groups of 16 rows in flight.
+template <int NB, int G = 1>
 __device__ __forceinline__ void warp_bf16_pairs(const DevView& v, const float* q, const uint32_t* ids, uint32_t cnt,
                                                 float* dout) {
     const int lane = threadIdx.x & 31, p = lane & 1;
-    for (uint32_t r = 0; r < cnt; r += 16) {
-        const uint32_t t = r + (lane >> 1);
-        const uint32_t id = ids[t < cnt ? t : r];
-        const float d = bf16_pair<NB>(q, v.vec_bf16 + (size_t)id * v.dim, p);
-        if (p == 0 && t < cnt) dout[t] = d;
+    for (uint32_t r = 0; r < cnt; r += 16 * G) {
+        Bf16Half<NB> h[G];
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+            if (g == 0 || r + 16 * g < cnt) {  // uniform over the warp
+                const uint32_t t = r + 16 * g + (lane >> 1);
+                h[g].load(v.vec_bf16 + (size_t)ids[t < cnt ? t : r] * (16 * NB), p);
+            }
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+            if (g == 0 || r + 16 * g < cnt) {
+                const uint32_t t = r + 16 * g + (lane >> 1);
+                const float d = h[g].dist(q, p);
+                if (p == 0 && t < cnt) dout[t] = d;
+            }
     }
 }
 
@@ -620,18 +641,21 @@ __device__ __forceinline__ void warp_bf16_pairs(const DevView& v, const float* q
 template <int DM, int RK = kRowsAny>
 __device__ __forceinline__ void warp_dist_list(const DevView& v, const float* q, const uint32_t* ids, uint32_t cnt,
                                                float* dout) {
-    if constexpr (DM == 3) {
+    if constexpr (DM == 3 && RK >= 64) {
         // q is the warp's s.q; its INT8 copy and (s_q^2 sum q8^2, s_q, e_q) follow it
+        warp_i8_rows<RK / 16>(v, i8_q_words(q, RK), *i8_q_meta(q, RK), ids, cnt, dout);
+        __syncwarp();
+    } else if constexpr (DM == 3) {
         warp_i8_list(v, i8_q_words(q, v.dim), *i8_q_meta(q, v.dim), ids, cnt, dout);
     } else if constexpr (DM < 2) {
         warp_l2_list<DM == 1, RK>(v, q, ids, cnt, dout);
     } else {
         const int lane = threadIdx.x & 31;
-        if (v.dim == 128) warp_bf16_pairs<8>(v, q, ids, cnt, dout);
-        else if (v.dim == 96) warp_bf16_pairs<6>(v, q, ids, cnt, dout);
-        else if (v.dim == 256) warp_bf16_pairs<16>(v, q, ids, cnt, dout);
-        else
+        if constexpr (RK >= 64) {
+            warp_bf16_pairs<RK / 16>(v, q, ids, cnt, dout);
+        } else {
             for (uint32_t t = lane; t < cnt; t += 32) dout[t] = bf16_thread(q, v.vec_bf16 + (size_t)ids[t] * v.dim, v.dim);
+        }
         __syncwarp();
     }
 }
@@ -642,6 +666,8 @@ __device__ __forceinline__ float warp_dist_one(const DevView& v, const float* q,
         return l2_half16<DM == 1>(q, v.vec + (size_t)id * v.dim, v.nb, threadIdx.x & 15);
     } else if constexpr (DM < 2) {
         return l2_thread(q, v.vec + (size_t)id * v.dim, v.dim, v.lanes, v.fused);
+    } else if constexpr (DM == 3 && RK >= 64) {
+        return i8_row<RK / 16>(i8_q_words(q, RK), *i8_q_meta(q, RK), v.vec_i8 + (size_t)id * RK, __ldg(v.i8_meta + id));
     } else if constexpr (DM == 3) {
         return i8_one(v, q, id);
     } else {
@@ -718,21 +744,26 @@ __device__ __forceinline__ uint32_t insert_pos(const float* td, uint32_t n, floa
 // whatever it would have moved.
 //
 // The beam is shifted 128 entries (four per lane) at a time from the right, each
-// entry by the number of insertion points at or before it: with few accepted
-// neighbours counting them costs less than a search per entry, and the four
-// entries' reads, counts and writes overlap.  (One 32-entry block at a time with a
+// entry by the number of insertion points at or before it: counting them costs less
+// than a search per entry, and the four entries' reads, counts and writes overlap.  (One 32-entry block at a time with a
 // binary search per entry, and shuffle loops for both rankings, took about two
 // thirds of the 8,000 cycles an expansion of a lone query cost at ef = 200.)
 //
 // known(d, ok, id, pos) is called by the whole warp once the neighbours to insert are
-// known (lanes with ok), before the beam changes.
-template <class F>
+// known (lanes with ok), before the beam changes.  DEDUP: an id may come twice (two
+// parents sharing a neighbour that the lossy visited cache did not catch): the lowest
+// lane keeps it.
+template <bool DEDUP = false, class F>
 __device__ __forceinline__ void beam_insert(WarpSmem& s, float d, uint32_t id, bool have, uint32_t EF, uint32_t& tsize,
                                             uint32_t& cursor, F&& known) {
     const int lane = threadIdx.x & 31;
     bool ok = have && !(tsize >= EF && d >= s.td[EF - 1]);
     uint32_t pos = 0, ab = __ballot_sync(0xFFFFFFFFu, ok);
     if (ab) {
+        if constexpr (DEDUP) {
+            const uint32_t same = __match_any_sync(0xFFFFFFFFu, ok ? id : kInvalid);
+            if (ok && (same & lanemask_lt() & ab)) ok = false;
+        }
         pos = insert_pos(s.td, tsize, d);
         if (ok) {
             for (int k = (int)pos - 1; k >= 0 && s.td[k] == d; --k)
@@ -745,14 +776,23 @@ __device__ __forceinline__ void beam_insert(WarpSmem& s, float d, uint32_t id, b
     }
     known(d, ok, id, pos);
     if (!ab) return;
-    const uint32_t na = __popc(ab);
+    const uint32_t na = __popc(ab), me = __popc(ab & lanemask_lt());
+    // ranks among the accepted ones, then their insertion points in that order, four
+    // at a time from shared memory (s.nd has been read: the callers hold d in registers)
+    const bool pad = (uint32_t)lane >= na && (uint32_t)lane < ((na + 3) & ~3u);
+    if (ok) s.nd[me] = d;
+    if (pad) s.nd[lane] = __uint_as_float(0x7F800000u);
+    __syncwarp();
     uint32_t before = 0;
-    for (uint32_t m = ab; m; m &= m - 1) {
-        const int i = __ffs(m) - 1;
-        const float di = __shfl_sync(0xFFFFFFFFu, d, i);
-        if (di < d || (di == d && i < lane)) before++;
+    for (uint32_t i = 0; i < na; i += 4) {
+        const float4 o = *reinterpret_cast<const float4*>(s.nd + i);
+        before += (uint32_t)(o.x < d || (o.x == d && i < me)) + (uint32_t)(o.y < d || (o.y == d && i + 1 < me)) +
+                  (uint32_t)(o.z < d || (o.z == d && i + 2 < me)) + (uint32_t)(o.w < d || (o.w == d && i + 3 < me));
     }
-    const uint32_t lo = __reduce_min_sync(0xFFFFFFFFu, ok ? pos : 0xFFFFFFFFu);
+    if (ok) s.apos[before] = pos;
+    if (pad) s.apos[lane] = 0xFFFFFFFFu;
+    __syncwarp();
+    const uint32_t lo = s.apos[0];
     const uint32_t newsize = min(tsize + na, EF);
     // every chunk is read before any lane writes, and its targets lie in itself or
     // in chunks to its right that were already moved
@@ -767,10 +807,13 @@ __device__ __forceinline__ void beam_insert(WarpSmem& s, float d, uint32_t id, b
                 ik[u] = k < tsize ? s.ti[k] : 0u;
                 np[u] = k < tsize ? k : 0xFFFF0000u;
             }
-            for (uint32_t m = ab; m; m &= m - 1) {
-                const uint32_t p = __shfl_sync(0xFFFFFFFFu, pos, __ffs(m) - 1);
+            for (uint32_t i = 0; i < na; i += 4) {
+                const uint4 p = *reinterpret_cast<const uint4*>(s.apos + i);
 #pragma unroll
-                for (int u = 0; u < 4; ++u) np[u] += p <= (uint32_t)b + 32 * u + lane ? 1u : 0u;
+                for (int u = 0; u < 4; ++u) {
+                    const uint32_t k = (uint32_t)b + 32 * u + lane;
+                    np[u] += (uint32_t)(p.x <= k) + (uint32_t)(p.y <= k) + (uint32_t)(p.z <= k) + (uint32_t)(p.w <= k);
+                }
             }
             __syncwarp();
 #pragma unroll

@@ -54,161 +54,87 @@ __device__ inline WarpSmem carve_fast(char* base, uint32_t dim, uint32_t efc, ui
     return s;
 }
 
-// ids[0..cnt) (cnt <= 64) scored with cooperative row reads (coop_i8_load): a
-// block of 32 rows in eight load rounds, four whole rows per load instruction.
-// R2: both blocks' loads issued before either is scored (one memory round trip
-// for 64 rows, twice the registers); otherwise block by block.
+// 32 rows' reads on their way, eight lanes per row (coop_i8_load): four whole rows per
+// load instruction; rows of 256 bytes in two halves.
+template <int NB>
+struct CoopRows {
+    static constexpr int H = NB > 8 ? 2 : 1;
+    int4 x[H][8];
+    float4 m;
+    __device__ __forceinline__ void load(const DevView& v, const uint32_t* ids, uint32_t b0, uint32_t cnt) {
+        const int g = (threadIdx.x >> 3) & 3;
+        const uint32_t r = coop_row();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t t = b0 + 4 * i + g;
+            const uint32_t id = ids[t < cnt ? t : 0];
+            if constexpr (H == 1) {
+                x[0][i] = coop_i8_load<NB>(v.vec_i8, id);
+            } else {
+                const int4* row = reinterpret_cast<const int4*>(v.vec_i8 + (size_t)id * (NB * 16)) + (threadIdx.x & 7);
+                x[0][i] = __ldg(row);
+                x[1][i] = __ldg(row + 8);
+            }
+        }
+        m = __ldg(v.i8_meta + ids[b0 + r < cnt ? b0 + r : 0]);
+    }
+    __device__ __forceinline__ void score(const int4 (&qw)[H], float4 qm, uint32_t b0, uint32_t cnt, float* dout) const {
+        int p[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            p[i] = dp4a4(x[0][i], qw[0]);
+            if constexpr (H == 2) p[i] += dp4a4(x[1][i], qw[1]);
+        }
+        const int d = coop_sum8(p);
+        const uint32_t r = coop_row();
+        if (b0 + r < cnt) dout[b0 + r] = qm.x + m.x * m.x * m.z - 2.f * qm.y * m.x * (float)d;
+    }
+};
+
+// ids[0..cnt) (cnt <= 64) scored with cooperative row reads, 32 at a time.  R2: both
+// blocks' loads issued before either is scored (one memory round trip for 64 rows,
+// twice the registers); otherwise block by block.
 template <int NB, bool R2>
 __device__ __forceinline__ void warp_i8_coop(const DevView& v, const int* q8, float4 qm, const uint32_t* ids,
                                              uint32_t cnt, float* dout) {
-    const int g = (threadIdx.x >> 3) & 3;
-    const int4 qw = coop_q_words<NB>(q8);
-    const uint32_t r = coop_row();
-    const uint32_t nb = cnt > 32 ? 2 : 1;
-    auto finish = [&](const int4 (&x)[8], float4 m, uint32_t b0) {
-        int p[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) p[i] = dp4a4(x[i], qw);
-        const int d = coop_sum8(p);
-        if (b0 + r < cnt) dout[b0 + r] = qm.x + m.x * m.x * m.z - 2.f * qm.y * m.x * (float)d;
-    };
+    int4 qw[CoopRows<NB>::H];
+    qw[0] = coop_q_words<(NB > 8 ? 8 : NB)>(q8);
+    if constexpr (NB > 8) qw[1] = coop_q_words<8>(q8 + 32);
     if constexpr (R2) {
-        int4 x0[8], x1[8];
-        float4 m0, m1 = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint32_t t = 4 * i + g;
-            x0[i] = coop_i8_load<NB>(v.vec_i8, ids[t < cnt ? t : 0]);
-        }
-        m0 = __ldg(v.i8_meta + ids[r < cnt ? r : 0]);
-        if (nb > 1) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const uint32_t t = 32 + 4 * i + g;
-                x1[i] = coop_i8_load<NB>(v.vec_i8, ids[t < cnt ? t : 0]);
-            }
-            m1 = __ldg(v.i8_meta + ids[32 + r < cnt ? 32 + r : 0]);
-        }
-        finish(x0, m0, 0);
-        if (nb > 1) finish(x1, m1, 32);
+        CoopRows<NB> a, b;
+        a.load(v, ids, 0, cnt);
+        if (cnt > 32) b.load(v, ids, 32, cnt);
+        a.score(qw, qm, 0, cnt, dout);
+        if (cnt > 32) b.score(qw, qm, 32, cnt, dout);
     } else {
-        for (uint32_t b0 = 0; b0 < 32 * nb; b0 += 32) {
-            int4 x[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const uint32_t t = b0 + 4 * i + g;
-                x[i] = coop_i8_load<NB>(v.vec_i8, ids[t < cnt ? t : 0]);
-            }
-            const float4 m = __ldg(v.i8_meta + ids[b0 + r < cnt ? b0 + r : 0]);
-            finish(x, m, b0);
+        for (uint32_t b0 = 0; b0 < cnt; b0 += 32) {
+            CoopRows<NB> a;
+            a.load(v, ids, b0, cnt);
+            a.score(qw, qm, b0, cnt, dout);
         }
     }
 }
 
 // Scores ids[0..cnt) (cnt <= 64) with the form's rows: DM 3 INT8, DM 2 BF16.
-// R2: all 64 INT8 rows in one memory round trip (at twice the registers and so
-// fewer resident warps) or 32 at a time; the launch-shape autotuner picks.
-template <int DM, bool R2>
+// R2: all 64 rows in one memory round trip (at more registers and so fewer resident
+// warps; two at 256 BF16 elements) or 32 INT8 / 16 BF16 rows at a time; the launch-shape
+// autotuner picks for INT8, and small batches, where latency counts, take R2.
+// RK: the width (0: any).
+template <int DM, bool R2, int RK>
 __device__ __forceinline__ void warp_dist_list64(const DevView& v, const float* q, const uint32_t* ids,
                                                  uint32_t cnt, float* dout) {
-    if constexpr (DM == 3) {
-        const int* q8 = i8_q_words(q, v.dim);
-        const float4 qm = *i8_q_meta(q, v.dim);
-        // rows of 96 and 128 bytes read cooperatively; other widths one row per
-        // lane, 32 at a time
-        const uint32_t nw = v.dim >> 4;
-        if (nw == 6) warp_i8_coop<6, R2>(v, q8, qm, ids, cnt, dout);
-        else if (nw == 8) warp_i8_coop<8, R2>(v, q8, qm, ids, cnt, dout);
-        else {
-            warp_i8_list(v, q8, qm, ids, min(cnt, 32u), dout);
-            if (cnt > 32) warp_i8_list(v, q8, qm, ids + 32, cnt - 32, dout + 32);
-        }
+    // INT8 rows of 96, 128 and 256 bytes read cooperatively; other widths one row per
+    // lane, 32 at a time
+    if constexpr (DM == 3 && RK >= 64) {
+        warp_i8_coop<RK / 16, R2>(v, i8_q_words(q, RK), *i8_q_meta(q, RK), ids, cnt, dout);
+        __syncwarp();
+    } else if constexpr (DM == 2 && RK >= 64 && R2) {
+        warp_bf16_pairs<RK / 16, RK <= 128 ? 4 : 2>(v, q, ids, cnt, dout);
         __syncwarp();
     } else {
-        warp_dist_list<DM>(v, q, ids, min(cnt, 32u), dout);
-        if (cnt > 32) warp_dist_list<DM>(v, q, ids + 32, cnt - 32, dout + 32);
+        warp_dist_list<DM, RK>(v, q, ids, min(cnt, 32u), dout);
+        if (cnt > 32) warp_dist_list<DM, RK>(v, q, ids + 32, cnt - 32, dout + 32);
     }
-}
-
-// Inserts the scored neighbours nd/ni[0..cnt) (cnt <= 32, one per lane) whose
-// distance is below a full beam's last entry; the beam stays sorted and is cut to
-// EF.  cursor moves back to the first inserted position.
-__device__ __forceinline__ void beam_insert_fast(WarpSmem& s, const float* nd, const uint32_t* ni, uint32_t cnt,
-                                                 uint32_t EF, uint32_t& tsize, uint32_t& cursor) {
-    const int lane = threadIdx.x & 31;
-    float d = FLT_MAX;
-    uint32_t id = kInvalid, pos = 0;
-    bool ok = false;
-    if ((uint32_t)lane < cnt) {
-        d = nd[lane];
-        id = ni[lane];
-        ok = !(tsize >= EF && d >= s.td[EF - 1]);
-    }
-    uint32_t okb = __ballot_sync(0xFFFFFFFFu, ok);
-    if (!okb) return;
-    // the same id twice in this batch (two parents sharing a neighbour that the
-    // lossy visited cache did not catch): the lowest lane keeps it
-    const uint32_t same = __match_any_sync(0xFFFFFFFFu, ok ? id : kInvalid);
-    if (ok && (same & lanemask_lt() & okb)) ok = false;
-    if (ok) {
-        pos = upper_bound(s.td, tsize, d);
-        for (int k = (int)pos - 1; k >= 0 && s.td[k] == d; --k)
-            if ((s.ti[k] & kIdMask) == id) {
-                ok = false;
-                break;
-            }
-    }
-    const uint32_t ab = __ballot_sync(0xFFFFFFFFu, ok);
-    if (!ab) return;
-    const uint32_t na = __popc(ab);
-    uint32_t before = 0;
-    if (na > 1) {
-        for (uint32_t m = ab; m; m &= m - 1) {
-            const int i = __ffs(m) - 1;
-            const float di = __shfl_sync(0xFFFFFFFFu, d, i);
-            if (di < d || (di == d && i < lane)) before++;
-        }
-    }
-    if (ok) s.apos[before] = pos;
-    __syncwarp();
-    const uint32_t lo = s.apos[0], amax = s.apos[na - 1];
-    const uint32_t newsize = min(tsize + na, EF);
-    if (tsize > lo) {
-        for (int b = (int)lo + (int)(((tsize - lo - 1) / 32) * 32); b >= (int)lo; b -= 32) {
-            const uint32_t k = (uint32_t)b + lane;
-            float dk = 0.f;
-            uint32_t ik = 0, np = 0xFFFFFFFFu;
-            if (k < tsize) {
-                dk = s.td[k];
-                ik = s.ti[k];
-                uint32_t sh = na;
-                if (k < amax) {
-                    uint32_t a = 0, e = na - 1;
-                    while (a < e) {
-                        const uint32_t mid = (a + e) >> 1;
-                        if (s.apos[mid] <= k) a = mid + 1;
-                        else e = mid;
-                    }
-                    sh = a;
-                }
-                np = k + sh;
-            }
-            __syncwarp();
-            if (np < newsize) {
-                s.td[np] = dk;
-                s.ti[np] = ik;
-            }
-            __syncwarp();
-        }
-    }
-    const uint32_t npos = pos + before;
-    if (ok && npos < newsize) {
-        s.td[npos] = d;
-        s.ti[npos] = id;
-    }
-    tsize = newsize;
-    cursor = min(cursor, lo);
-    __syncwarp();
 }
 
 // Two-parent search of level 0 continuing from the beam s.td/s.ti[0..tsize)
@@ -217,7 +143,7 @@ __device__ __forceinline__ void beam_insert_fast(WarpSmem& s, const float* nd, c
 // (<= EF) are expanded, the rest is a reserve a later search with a larger beam
 // can resume from (the first EX entries evolve exactly as in a search with
 // EF = EX).  Returns the beam size (<= EF).
-template <int DM, bool R2>
+template <int DM, bool R2, int RK>
 __device__ uint32_t beam_search_fast(const DevView& v, WarpSmem& s, uint32_t tsize, uint32_t EF, uint32_t EX,
                                      uint32_t vc, unsigned long long& c_dist, unsigned long long& c_exp) {
     const int lane = threadIdx.x & 31;
@@ -274,10 +200,13 @@ __device__ uint32_t beam_search_fast(const DevView& v, WarpSmem& s, uint32_t tsi
             __syncwarp();
         }
         if (cnt == 0) continue;
-        warp_dist_list64<DM, R2>(v, s.q, s.ni, cnt, s.nd);
+        warp_dist_list64<DM, R2, RK>(v, s.q, s.ni, cnt, s.nd);
         c_dist += cnt;
-        beam_insert_fast(s, s.nd, s.ni, min(cnt, 32u), EF, tsize, cursor);
-        if (cnt > 32) beam_insert_fast(s, s.nd + 32, s.ni + 32, cnt - 32, EF, tsize, cursor);
+        for (uint32_t b = 0; b < cnt; b += 32) {
+            const bool have = b + lane < cnt;
+            beam_insert<true>(s, have ? s.nd[b + lane] : FLT_MAX, have ? s.ni[b + lane] : kInvalid, have, EF, tsize,
+                              cursor, [](float, bool, uint32_t, uint32_t) {});
+        }
     }
     return tsize;
 }

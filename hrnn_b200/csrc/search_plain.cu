@@ -163,8 +163,17 @@ __global__ void __launch_bounds__(T == 1 ? 128 : 32 * T, T == 1 ? 4 : RK == 64 |
 //   resume: start from the stored beam instead of the descent (its ids seed the
 //     visited cache), continue with the query's own ef, store nothing;
 //   nq_dev: as k_phase_a.
-template <int DM, bool R2>
-__global__ void __launch_bounds__(128, R2 ? 4 : 1) k_phase_a_fast(DevView v, const float* __restrict__ Q, uint32_t nq,
+// RK: the width 96, 128 or 256, else 0 (with one kernel for all widths the widest
+// one's rows set the registers: 144 for INT8, three blocks per SM).  Blocks per SM the
+// registers are cut to, of the 1M x 128 INT8 plan: 4 4.16 ms, 5 3.84, 6 3.82, 7 3.69, 8
+// 3.71; BF16 rows want their loads in flight more than more warps.
+template <int DM, bool R2, int RK>
+constexpr int fast_blocks() {
+    return DM == 2 || RK == 0 ? 1 : R2 ? (RK == 256 ? 3 : 4) : RK == 256 ? 4 : 7;
+}
+
+template <int DM, bool R2, int RK>
+__global__ void __launch_bounds__(128, fast_blocks<DM, R2, RK>()) k_phase_a_fast(DevView v, const float* __restrict__ Q, uint32_t nq,
                                                       const uint32_t* __restrict__ qm,
                                                       const uint32_t* __restrict__ qef, uint32_t efc, uint32_t vc,
                                                       uint32_t mmax, uint32_t* __restrict__ prox,
@@ -208,9 +217,9 @@ __global__ void __launch_bounds__(128, R2 ? 4 : 1) k_phase_a_fast(DevView v, con
             __syncwarp();
         } else {
             uint32_t cur = v.enterpoint;
-            float curd = warp_dist_one<DM>(v, s.q, cur);
+            float curd = warp_dist_one<DM, RK>(v, s.q, cur);
             c_dist++;
-            greedy_descent<DM, kRowsAny>(v, s, v.maxlevel, 0, cur, curd, c_dist);
+            greedy_descent<DM, RK>(v, s, v.maxlevel, 0, cur, curd, c_dist);
             if (lane == 0) {
                 s.td[0] = curd;
                 s.ti[0] = cur;
@@ -222,7 +231,7 @@ __global__ void __launch_bounds__(128, R2 ? 4 : 1) k_phase_a_fast(DevView v, con
         // a frontier pass that stores its beam keeps a reserve beyond EF for the
         // resumed search (expanding only the first EF entries)
         const uint32_t cap_beam = (save_cap && !resume) ? max(EF, min(save_cap, efc)) : EF;
-        tsize = beam_search_fast<DM, R2>(v, s, tsize, cap_beam, EF, vc, c_dist, c_exp);
+        tsize = beam_search_fast<DM, R2, RK>(v, s, tsize, cap_beam, EF, vc, c_dist, c_exp);
         if (save_cap && !resume) {
             const uint32_t ns = min(tsize, save_cap);
             for (uint32_t i = lane; i < ns; i += 32) {
@@ -535,6 +544,10 @@ using KPhaseA = void (*)(DevView, const float*, uint32_t, const uint32_t*, const
                          uint32_t*, uint32_t*, SearchCounters*, const uint32_t*, uint32_t, uint32_t, uint32_t, float*,
                          uint32_t*, const uint32_t*);
 
+// Up to this many queries the reduced-precision search spreads its warps over the SMs,
+// one block each, with as many rows in flight as a step has.
+static size_t fast_spread(int nsm) { return (size_t)nsm * 4; }
+
 // Whether a batch gets a team of warps per query (exact forms): too few queries to
 // fill the device, and link rows and beam as beam_search_team takes them.
 static bool phase_a_team(bool fast, int dm, const DevView& v, size_t nq, uint32_t efc, int nsm) {
@@ -554,10 +567,28 @@ static KPhaseA phase_a_exact(int dm, const DevView& v, bool team) {
     });
 }
 
+using KPhaseAFast = void (*)(DevView, const float*, uint32_t, const uint32_t*, const uint32_t*, uint32_t, uint32_t,
+                             uint32_t, uint32_t*, uint32_t*, SearchCounters*, const uint32_t*, uint32_t, uint32_t,
+                             uint32_t, float*, uint32_t*, uint32_t, uint32_t*, float*, uint32_t*, int,
+                             const uint32_t*);
+
+// The two-parent kernel of a distance mode and width.
+static KPhaseAFast phase_a_fast(int dm, bool r2, uint32_t dim) {
+    auto of = [&](auto rk) -> KPhaseAFast {
+        constexpr int RK = decltype(rk)::value;
+        if (dm == 3) return r2 ? k_phase_a_fast<3, true, RK> : k_phase_a_fast<3, false, RK>;
+        return r2 ? k_phase_a_fast<2, true, RK> : k_phase_a_fast<2, false, RK>;
+    };
+    switch (dim) {
+        case 96: return of(std::integral_constant<int, 96>{});
+        case 128: return of(std::integral_constant<int, 128>{});
+        case 256: return of(std::integral_constant<int, 256>{});
+        default: return of(std::integral_constant<int, 0>{});
+    }
+}
+
 static const void* phase_a_kernel(bool fast, int dm, bool r2, const DevView& v, bool team) {
-    return fast ? (dm == 3 ? (r2 ? (const void*)k_phase_a_fast<3, true> : (const void*)k_phase_a_fast<3, false>)
-                           : (const void*)k_phase_a_fast<2, false>)
-                : (const void*)phase_a_exact(dm, v, team);
+    return fast ? (const void*)phase_a_fast(dm, r2, v.dim) : (const void*)phase_a_exact(dm, v, team);
 }
 
 // One launch; qlist / m_over / ef_over / m_keep / proxd / save / resume / nq_dev as
@@ -567,8 +598,7 @@ static void launch_phase_a(const PhaseA& p, unsigned g, int cw, uint32_t cv, siz
                     uint32_t* ctrq, uint32_t save_cap, uint32_t* st_cnt, float* st_d, uint32_t* st_i, int resume,
                     const uint32_t* nq_dev) {
     if (p.fast) {
-        auto k = p.dm == 3 ? (p.r2 ? k_phase_a_fast<3, true> : k_phase_a_fast<3, false>) : k_phase_a_fast<2, false>;
-        k<<<g, cw * 32, sm, ls>>>(p.v, p.q, nqq, p.qm, p.qef, p.efc, cv, p.mmax, p.prox, p.nprox, p.ctr, qlist, m_over,
+        phase_a_fast(p.dm, p.r2, p.v.dim)<<<g, cw * 32, sm, ls>>>(p.v, p.q, nqq, p.qm, p.qef, p.efc, cv, p.mmax, p.prox, p.nprox, p.ctr, qlist, m_over,
                                   ef_over, m_keep, proxd, ctrq, save_cap, st_cnt, st_d, st_i, resume, nq_dev);
     } else {
         phase_a_exact(p.dm, p.v, p.team)<<<g, cw * 32, sm, ls>>>(p.v, p.q, nqq, p.qm, p.qef, p.efc, cv, p.mmax, p.prox, p.nprox, p.ctr, qlist, m_over,
@@ -701,6 +731,9 @@ uint64_t search_batch(Index& ix, const SearchArgs& a) {
         auto shape = ix.autotune ? ix.a_shape.find(shape_key) : ix.a_shape.end();
         if (team) {
             wpb = kTeamWarps;
+        } else if (fast && nq <= fast_spread(nsm)) {
+            wpb = 1;
+            r2 = true;
         } else if (shape != ix.a_shape.end()) {
             wpb = (int)(shape->second.first & 0xFF);
             r2 = (shape->second.first & 0x100) != 0;
@@ -1063,7 +1096,7 @@ void budget_features(Index& ix, const float* d_q, size_t nq, uint32_t k, uint32_
     const int nsm = sms(ix.device);
     unsigned grid = (unsigned)std::max<size_t>(1, std::min<size_t>((nq + wpb - 1) / wpb, (size_t)nsm * 16));
     if (fast) {
-        auto kern = int8 ? k_phase_a_fast<3, false> : k_phase_a_fast<2, false>;
+        auto kern = phase_a_fast(int8 ? 3 : 2, false, v.dim);
         CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
         kern<<<grid, wpb * 32, smem_a, s>>>(v, d_q, (uint32_t)nq, nullptr, nullptr, efc, vc, mmax,
                                             prox.as<uint32_t>(), nprox.as<uint32_t>(),
@@ -1145,6 +1178,12 @@ PlanLaunch plan_launch_shape(Index& ix, const SearchPlan& p) {
         L.smem_a = wsm_of(L.vc) * L.wpb;
     }
     L.team = !L.learned && phase_a_team(L.fast, dm, v, p.nq, L.efc, sms(ix.device));
+    if (L.fast && p.nq <= fast_spread(sms(ix.device))) {
+        L.wpb = 1;
+        L.r2 = true;
+        L.vc = 512;
+        L.smem_a = wsm_of(L.vc);
+    }
     if (L.team) {
         L.wpb = kTeamWarps;
         L.vc = team_vis(L.efc);
