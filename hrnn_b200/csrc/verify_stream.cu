@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "beam.cuh"
+#include "csr_kernels.cuh"
 #include "index.hpp"
 #include "verify_stream.hpp"
 
@@ -32,7 +33,7 @@ namespace hrnn {
 namespace {
 
 constexpr uint32_t kChunk = 256;     // postings per work item
-constexpr uint32_t kFinCap = 1024;   // acceptances a query's finishing warp sorts in shared memory
+constexpr uint32_t kFinCap = 1024;   // acceptances a query's finishing warp sorts in registers
 constexpr uint32_t kBigCap = 16384;  // ... and a finishing block (64 KB of shared memory)
 constexpr float kTieUlpsS = 16.f;    // FP64 re-decision band around the radius, in ulps of kd
 
@@ -351,52 +352,62 @@ __global__ void __launch_bounds__(256, verify_min_blocks<S>()) k_verify_chunks(
     }
 }
 
-// One warp per query: sort the accepted ids (bitonic, shared memory), drop
-// repeats, write the labels over the query's slice; queries with more than
-// kFinCap acceptances are listed for k_stream_finish_big.
-__global__ void __launch_bounds__(256) k_stream_finish(DevView v, uint32_t nq, const uint64_t* __restrict__ res_off,
+// The warp's 32 R ids (kInvalid beyond na) sorted, repeats dropped, the labels of the
+// others written to out[0..); returns their number.
+template <int R>
+__device__ __forceinline__ uint32_t finish_ids(const DevView& v, uint64_t* __restrict__ out, uint32_t na) {
+    const int lane = threadIdx.x & 31;
+    uint32_t x[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) x[r] = 32 * r + lane < na ? (uint32_t)out[32 * r + lane] : kInvalid;
+    warp_sort<uint32_t, R>(x);
+    uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, x[R - 1], 1), mine = 0;  // id lane R + r in x[r]
+    bool keep[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        keep[r] = x[r] != kInvalid && (x[r] != prev || (r == 0 && lane == 0));
+        prev = x[r];
+        mine += keep[r] ? 1u : 0u;
+    }
+    uint32_t incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    uint32_t at = incl - mine;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        if (keep[r]) out[at++] = v.labels[x[r]];
+    return __shfl_sync(0xFFFFFFFFu, incl, 31);
+}
+
+// One warp per query: the accepted ids sorted in registers, repeats dropped, the
+// labels written over the query's slice; queries with more than kFinCap acceptances
+// are listed for k_stream_finish_big.
+__global__ void __launch_bounds__(128) k_stream_finish(DevView v, uint32_t nq, const uint64_t* __restrict__ res_off,
                                                        const uint32_t* __restrict__ acc_cnt,
                                                        uint64_t* __restrict__ resbuf, uint32_t* __restrict__ res_count,
                                                        uint32_t* __restrict__ big, uint32_t* __restrict__ n_big,
                                                        SearchCounters* __restrict__ ctr,
                                                        const uint8_t* __restrict__ grp, uint8_t want) {
-    __shared__ uint32_t sm[8][kFinCap];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t qi = blockIdx.x * 8 + w;
+    const uint32_t qi = blockIdx.x * 4 + w;
     if (qi >= nq || (grp && grp[qi] != want)) return;
-    uint32_t* acc = sm[w];
     const uint32_t na = acc_cnt[qi];
-    if (na > kFinCap || na > res_off[qi + 1] - res_off[qi]) {  // left to the block-wide pass
+    const uint64_t ro = res_off[qi];
+    if (na > kFinCap || na > res_off[qi + 1] - ro) {  // left to the block-wide pass
         if (lane == 0) big[atomicAdd(n_big, 1u)] = qi;
         return;
     }
-    const uint64_t ro = res_off[qi];
-    uint32_t P = 32;
-    while (P < na) P <<= 1;
-    for (uint32_t i = lane; i < P; i += 32) acc[i] = i < na ? (uint32_t)resbuf[ro + i] : kInvalid;
-    __syncwarp();
-    for (uint32_t k = 2; k <= P; k <<= 1)
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t i = lane; i < P; i += 32) {
-                const uint32_t y = i ^ j;
-                if (y > i) {
-                    const uint32_t a0 = acc[i], a1 = acc[y];
-                    if ((a0 > a1) == ((i & k) == 0)) {
-                        acc[i] = a1;
-                        acc[y] = a0;
-                    }
-                }
-            }
-            __syncwarp();
-        }
+    uint64_t* out = resbuf + ro;
     uint32_t nu = 0;
-    for (uint32_t b0 = 0; b0 < na; b0 += 32) {
-        const uint32_t i = b0 + lane;
-        const bool keep = i < na && (i == 0 || acc[i] != acc[i - 1]);
-        const uint32_t kb = __ballot_sync(0xFFFFFFFFu, keep);
-        if (keep) resbuf[ro + nu + __popc(kb & ((1u << lane) - 1u))] = v.labels[acc[i]];
-        nu += __popc(kb);
-    }
+    if (na <= 32) nu = finish_ids<1>(v, out, na);
+    else if (na <= 64) nu = finish_ids<2>(v, out, na);
+    else if (na <= 128) nu = finish_ids<4>(v, out, na);
+    else if (na <= 256) nu = finish_ids<8>(v, out, na);
+    else if (na <= 512) nu = finish_ids<16>(v, out, na);
+    else nu = finish_ids<32>(v, out, na);
     if (lane == 0) {
         res_count[qi] = nu;
         if (nu) atomicAdd(&ctr->n_result, (unsigned long long)nu);
@@ -417,7 +428,7 @@ __global__ void __launch_bounds__(1024) k_stream_finish_big(DevView v, const uin
                                                             uint32_t* __restrict__ ovl, uint32_t* __restrict__ n_ovl,
                                                             SearchCounters* __restrict__ ctr) {
     extern __shared__ uint32_t acc[];  // kBigCap
-    __shared__ uint32_t ctl[2];
+    __shared__ uint32_t ctl[2], wsum[32];
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t nb = *n_big;
     for (;;) {
@@ -451,19 +462,30 @@ __global__ void __launch_bounds__(1024) k_stream_finish_big(DevView v, const uin
                 }
                 __syncthreads();
             }
-        if (tid < 32) {  // one warp compacts the sorted ids
-            uint32_t nu = 0;
-            for (uint32_t b0 = 0; b0 < na; b0 += 32) {
-                const uint32_t i = b0 + lane;
-                const bool keep = i < na && (i == 0 || acc[i] != acc[i - 1]);
-                const uint32_t kb = __ballot_sync(0xFFFFFFFFu, keep);
-                if (keep) resbuf[ro + nu + __popc(kb & ((1u << lane) - 1u))] = v.labels[acc[i]];
-                nu += __popc(kb);
+        // the block compacts the sorted ids, 1024 at a time (one warp going through
+        // them alone, a label read a step, took as long as the sort)
+        uint32_t nu = 0;
+        for (uint32_t b0 = 0; b0 < na; b0 += blockDim.x) {
+            const uint32_t i = b0 + tid;
+            const bool keep = i < na && (i == 0 || acc[i] != acc[i - 1]);
+            const uint32_t kb = __ballot_sync(0xFFFFFFFFu, keep);
+            if (lane == 0) wsum[tid >> 5] = __popc(kb);
+            __syncthreads();
+            const uint32_t mine = wsum[lane];
+            uint32_t incl = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                if (lane >= o) incl += y;
             }
-            if (lane == 0) {
-                res_count[qi] = nu;
-                if (nu) atomicAdd(&ctr->n_result, (unsigned long long)nu);
-            }
+            const uint32_t before = __shfl_sync(0xFFFFFFFFu, incl - mine, tid >> 5);
+            if (keep) resbuf[ro + nu + before + __popc(kb & ((1u << lane) - 1u))] = v.labels[acc[i]];
+            nu += __shfl_sync(0xFFFFFFFFu, incl, 31);
+            __syncthreads();  // wsum is free again
+        }
+        if (tid == 0) {
+            res_count[qi] = nu;
+            if (nu) atomicAdd(&ctr->n_result, (unsigned long long)nu);
         }
     }
 }
@@ -593,7 +615,7 @@ void stream_verify(const DevView& v, bool wide, bool fused, const float* Q, uint
     else go(std::integral_constant<int, 2>{});
     uint32_t* big_n = B.ctl.as<uint32_t>() + 2;  // [2] big queries, [3] their work counter
     uint32_t* big = B.acc_cnt.as<uint32_t>() + nq;
-    k_stream_finish<<<(nq + 7) / 8, 256, 0, s>>>(v, nq, res_off, B.acc_cnt.as<uint32_t>(), resbuf, res_count, big,
+    k_stream_finish<<<(nq + 3) / 4, 128, 0, s>>>(v, nq, res_off, B.acc_cnt.as<uint32_t>(), resbuf, res_count, big,
                                                  big_n, ctr, grp, want);
     CUDA_LAUNCH_CHECK();
     k_stream_finish_big<<<nsm, 1024, kBigCap * 4, s>>>(v, res_off, B.acc_cnt.as<uint32_t>(), big, big_n, big_n + 1,
