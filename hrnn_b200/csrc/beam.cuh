@@ -328,7 +328,7 @@ __device__ __forceinline__ void warp_l2_list(const DevView& v, const float* q, c
         for (uint32_t t = threadIdx.x & 31; t < cnt; t += 32)
             dout[t] = l2_thread(q, v.vec + (size_t)ids[t] * v.dim, v.dim, v.lanes, v.fused);
     } else {
-        warp_l2_quads<FUSED, RK / 16, RK <= 128 ? 2 : 1>(v, q, ids, cnt, dout);
+        warp_l2_quads<FUSED, RK / 16, 1>(v, q, ids, cnt, dout);
     }
     __syncwarp();
 }

@@ -41,43 +41,6 @@ __device__ __forceinline__ uint32_t owner_of(const void* ent, uint64_t i, uint32
     return (uint32_t)(((const E*)ent)[i] >> rb);
 }
 
-// Two exact distances per half-warp with the loads of both vectors in flight.
-template <bool FUSED>
-__device__ __forceinline__ void l2_half16_x2(const float* __restrict__ q, const float* __restrict__ x0,
-                                             const float* __restrict__ x1, uint32_t nb, int l, float& d0,
-                                             float& d1) {
-    float a0 = 0.f, a1 = 0.f;
-    uint32_t i = 0;
-    for (; i + 4 <= nb; i += 4) {
-        float u0 = __ldg(x0 + 16 * (i + 0) + l), u1 = __ldg(x0 + 16 * (i + 1) + l);
-        float u2 = __ldg(x0 + 16 * (i + 2) + l), u3 = __ldg(x0 + 16 * (i + 3) + l);
-        float w0 = __ldg(x1 + 16 * (i + 0) + l), w1 = __ldg(x1 + 16 * (i + 1) + l);
-        float w2 = __ldg(x1 + 16 * (i + 2) + l), w3 = __ldg(x1 + 16 * (i + 3) + l);
-        float q0 = q[16 * (i + 0) + l], q1 = q[16 * (i + 1) + l], q2 = q[16 * (i + 2) + l], q3 = q[16 * (i + 3) + l];
-        a0 = sq_step(a0, q0 - u0, FUSED);
-        a1 = sq_step(a1, q0 - w0, FUSED);
-        a0 = sq_step(a0, q1 - u1, FUSED);
-        a1 = sq_step(a1, q1 - w1, FUSED);
-        a0 = sq_step(a0, q2 - u2, FUSED);
-        a1 = sq_step(a1, q2 - w2, FUSED);
-        a0 = sq_step(a0, q3 - u3, FUSED);
-        a1 = sq_step(a1, q3 - w3, FUSED);
-    }
-    for (; i < nb; ++i) {
-        float qq = q[16 * i + l];
-        a0 = sq_step(a0, qq - __ldg(x0 + 16 * i + l), FUSED);
-        a1 = sq_step(a1, qq - __ldg(x1 + 16 * i + l), FUSED);
-    }
-    float s0 = __shfl_sync(0xFFFFFFFFu, a0, 0, 16), s1 = __shfl_sync(0xFFFFFFFFu, a1, 0, 16);
-#pragma unroll
-    for (int k = 1; k < 16; ++k) {
-        s0 = __fadd_rn(s0, __shfl_sync(0xFFFFFFFFu, a0, k, 16));
-        s1 = __fadd_rn(s1, __shfl_sync(0xFFFFFFFFu, a1, k, 16));
-    }
-    d0 = s0;
-    d1 = s1;
-}
-
 }  // namespace
 
 __global__ void k_kdist_column(DevView v, uint32_t kidx, float* __restrict__ kcol) {
@@ -96,17 +59,18 @@ __global__ void k_kdist_column(DevView v, uint32_t kidx, float* __restrict__ kco
 __host__ __device__ constexpr uint32_t table_max(bool, bool) { return 8192; }
 
 // dynamic shared memory: q[dim] | keys[H] | cnt[H] (threshold > 1 only) |
-// stage[warps][32] | acc[kACap] | ctl[16] | q8 (dim bytes, padded to 16) | qm,
+// stage[warps][64] | acc[kACap] | dists[warps][32] | ctl[16] | q8 (dim bytes, padded to 16) | qm,
 // H = table_max(counts, mixed)
 __host__ size_t bc_cta_smem(uint32_t dim, bool counts, bool mixed) {
     const size_t H = table_max(counts, mixed);
-    return (size_t)dim * 4 + H * 4 + (counts ? H * 4 : 0) + (kBCThreads / 32) * 64 * 4 + (size_t)kACap * 4 + 64 +
+    return (size_t)dim * 4 + H * 4 + (counts ? H * 4 : 0) + (kBCThreads / 32) * 96 * 4 + (size_t)kACap * 4 + 64 +
            (((size_t)dim + 15) & ~(size_t)15) + 16;
 }
 
 constexpr float kTieUlps = 16.f;  // FP64 re-decision band around the radius, in ulps of kd
 
-template <class E, bool FUSED, bool COUNTS, bool MIXED>
+// RK: how the exact forms read rows (beam.cuh; 0 for the mixed ones).
+template <class E, bool FUSED, bool COUNTS, bool MIXED, int RK>
 __global__ void __launch_bounds__(kBCThreads) k_phase_bc_cta(
     DevView v, const float* __restrict__ Q, uint32_t nq, uint32_t mmax, const uint32_t* __restrict__ prox,
     const uint32_t* __restrict__ nprox, const uint32_t* __restrict__ plen, const uint64_t* __restrict__ qtotal,
@@ -123,12 +87,12 @@ __global__ void __launch_bounds__(kBCThreads) k_phase_bc_cta(
     uint32_t* cnt = keys + HM;
     uint32_t* stage = COUNTS ? cnt + HM : cnt;
     uint32_t* acc = stage + NW * 64;
-    uint32_t* ctl = acc + kACap;  // 0: query, 1: accepted count, 2: overflow, 3: table full
+    float* dists = (float*)(acc + kACap);  // a warp's distances
+    uint32_t* ctl = (uint32_t*)(dists + NW * 32);  // 0: query, 1: accepted count, 2: overflow, 3: table full
     int* q8 = (int*)(ctl + 16);   // INT8 screen: the query as packed int8 words
     float4* qm = (float4*)((char*)q8 + ((v.dim + 15) & ~15u));  // (s_q^2 sum q8^2, s_q, ||q - s_q q8||, 0)
     const bool i8s = MIXED && v.i8_screen && v.vec_i8 != nullptr;
     unsigned long long c_post = 0, c_cand = 0, c_ver = 0, c_res = 0;
-    const bool fast = v.lanes == 16 && (v.dim % 16) == 0;
     for (;;) {
         __syncthreads();
         if (tid == 0) ctl[0] = atomicAdd(next_q, 1u);
@@ -229,23 +193,11 @@ __global__ void __launch_bounds__(kBCThreads) k_phase_bc_cta(
             // Candidates are staged per warp until 32 are ready, then verified one
             // row per lane (32 rows in flight per warp).
             uint32_t* st = stage + w * 64;
+            float* dl = dists + w * 32;
             uint32_t ns = 0;
             auto accept = [&](uint32_t id) {
                 const uint32_t pos = atomicAdd(&ctl[1], 1u);
                 if (pos < kACap) acc[pos] = id;
-            };
-            // two lanes per row for the common dims (one memory round trip per 16
-            // rows), one row per lane otherwise
-            auto verify_pairs = [&](uint32_t cnt_, auto nbc) {
-                constexpr int NB = decltype(nbc)::value;
-                const int p = lane & 1;
-                for (uint32_t r = 0; r < cnt_; r += 16) {
-                    const uint32_t t = r + (lane >> 1);
-                    const uint32_t id = st[t < cnt_ ? t : r];
-                    const float kd = __ldg(kcol + id);
-                    const float d = l2_pair16<FUSED, NB>(q, v.vec + (size_t)id * v.dim, p);
-                    if (p == 0 && t < cnt_ && d <= kd) accept(id);
-                }
             };
             // Mixed precision: a BF16 screen decides whatever its error bound allows;
             // the rest is decided in exact FP32 (the reference's order), and inside a
@@ -356,23 +308,14 @@ __global__ void __launch_bounds__(kBCThreads) k_phase_bc_cta(
                     if (v.dim == 128) verify_mixed(cnt_, std::integral_constant<int, 8>{});
                     else if (v.dim == 96) verify_mixed(cnt_, std::integral_constant<int, 6>{});
                     else if (v.dim == 256) verify_mixed(cnt_, std::integral_constant<int, 16>{});
-                    else verify_pairs(cnt_, std::integral_constant<int, 8>{});  // unreachable: mixed needs 96/128/256
                     __syncwarp();
                     return;
                 }
-                if (fast && v.dim == 128) {
-                    verify_pairs(cnt_, std::integral_constant<int, 8>{});
-                } else if (fast && v.dim == 96) {
-                    verify_pairs(cnt_, std::integral_constant<int, 6>{});
-                } else if (fast && v.dim == 256) {
-                    verify_pairs(cnt_, std::integral_constant<int, 16>{});
-                } else if ((uint32_t)lane < cnt_) {
-                    const uint32_t id = st[lane];
-                    const float kd = __ldg(kcol + id);
-                    const float* x = v.vec + (size_t)id * v.dim;
-                    const float d = fast ? l2_row16<FUSED>(q, x, v.nb) : l2_thread(q, x, v.dim, v.lanes, v.fused);
-                    if (d <= kd) accept(id);
-                }
+                // exact FP32, four lanes per row (eight rows in a load instruction, half
+                // the lines of two lanes per row): the distances go through shared memory
+                // to the lane of each row
+                warp_l2_list<FUSED, RK>(v, q, st, cnt_, dl);
+                if ((uint32_t)lane < cnt_ && dl[lane] <= __ldg(kcol + st[lane])) accept(st[lane]);
                 __syncwarp();
             };
             for (uint32_t base = w * 32; base < HS; base += NW * 32) {
@@ -460,12 +403,18 @@ __global__ void __launch_bounds__(kBCThreads) k_phase_bc_cta(
 }
 
 // explicit instantiations used by search_plain.cu
-#define INST(E, F, C, X)                                                                                            \
-    template __global__ void k_phase_bc_cta<E, F, C, X>(DevView, const float*, uint32_t, uint32_t, const uint32_t*, \
-                                                        const uint32_t*, const uint32_t*, const uint64_t*,          \
-                                                        const uint64_t*, float, const float*, uint32_t, uint64_t*,  \
-                                                        uint32_t*, uint32_t*, uint32_t*, uint32_t*, SearchCounters*);
-#define INST2(E, F, C) INST(E, F, C, false) INST(E, F, C, true)
+#define INST(E, F, C, X, R)                                                                                        \
+    template __global__ void k_phase_bc_cta<E, F, C, X, R>(DevView, const float*, uint32_t, uint32_t, const uint32_t*, \
+                                                           const uint32_t*, const uint32_t*, const uint64_t*,      \
+                                                           const uint64_t*, float, const float*, uint32_t, uint64_t*, \
+                                                           uint32_t*, uint32_t*, uint32_t*, uint32_t*, SearchCounters*);
+#define INST2(E, F, C)                                                                                             \
+    INST(E, F, C, true, 0)                                                                                         \
+    INST(E, F, C, false, 64)                                                                                       \
+    INST(E, F, C, false, 96)                                                                                       \
+    INST(E, F, C, false, 128)                                                                                      \
+    INST(E, F, C, false, 256)                                                                                      \
+    INST(E, F, C, false, kRows16) INST(E, F, C, false, kRows4) INST(E, F, C, false, kRowsAny)
 INST2(uint32_t, false, false)
 INST2(uint32_t, false, true)
 INST2(uint32_t, true, false)

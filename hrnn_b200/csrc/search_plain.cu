@@ -30,20 +30,25 @@
 namespace hrnn {
 
 // search_bc.cu
-template <class E, bool FUSED, bool COUNTS, bool MIXED>
+template <class E, bool FUSED, bool COUNTS, bool MIXED, int RK>
 __global__ void k_phase_bc_cta(DevView, const float*, uint32_t, uint32_t, const uint32_t*, const uint32_t*,
                                const uint32_t*, const uint64_t*, const uint64_t*, float, const float*, uint32_t,
                                uint64_t*, uint32_t*, uint32_t*, uint32_t*, uint32_t*, SearchCounters*);
 using KCta = void (*)(DevView, const float*, uint32_t, uint32_t, const uint32_t*, const uint32_t*, const uint32_t*,
                       const uint64_t*, const uint64_t*, float, const float*, uint32_t, uint64_t*, uint32_t*,
                       uint32_t*, uint32_t*, uint32_t*, SearchCounters*);
+// The verification kernel of an order (f: fused), a threshold above 1 (c), the mixed
+// forms (x) and the view's rows (the exact forms).
 template <class E>
-KCta pick_bc(bool f, bool c, bool x) {
+KCta pick_bc(bool f, bool c, bool x, const DevView& v) {
     if (x)
-        return f ? (c ? k_phase_bc_cta<E, true, true, true> : k_phase_bc_cta<E, true, false, true>)
-                 : (c ? k_phase_bc_cta<E, false, true, true> : k_phase_bc_cta<E, false, false, true>);
-    return f ? (c ? k_phase_bc_cta<E, true, true, false> : k_phase_bc_cta<E, true, false, false>)
-             : (c ? k_phase_bc_cta<E, false, true, false> : k_phase_bc_cta<E, false, false, false>);
+        return f ? (c ? k_phase_bc_cta<E, true, true, true, 0> : k_phase_bc_cta<E, true, false, true, 0>)
+                 : (c ? k_phase_bc_cta<E, false, true, true, 0> : k_phase_bc_cta<E, false, false, true, 0>);
+    return with_rows(rows_kind(v.dim, v.lanes), [&](auto rk) -> KCta {
+        constexpr int RK = decltype(rk)::value;
+        return f ? (c ? k_phase_bc_cta<E, true, true, false, RK> : k_phase_bc_cta<E, true, false, false, RK>)
+                 : (c ? k_phase_bc_cta<E, false, true, false, RK> : k_phase_bc_cta<E, false, false, false, RK>);
+    });
 }
 void ensure_bf16(Index& ix);  // mixed.cu
 void ensure_i8(Index& ix);    // mixed.cu
@@ -74,11 +79,19 @@ namespace {
 
 // DM: distance mode of beam.cuh (0/1 exact FP32 unfused/fused, 2 BF16 rows, 3
 // INT8 rows against the INT8-quantised query).
+// Blocks per SM the registers are cut to.  10,000 queries on 300k x 128: 4 blocks with
+// sixteen rows in flight per warp 5.52 ms; eight rows in flight and 4 blocks 4.99, 5
+// 4.58, 6 4.28, 8 4.90.  6 is best at 64, 96, 256 and 272 too; widths read by quads of
+// single elements spill there (6,000 queries at d = 100: 4 3.01 ms, 6 4.29).
+constexpr int phase_a_blocks(int rk, int t) {
+    return t == 1 ? (rk == kRows4 ? 4 : 6) : rk == 64 || rk == kRows4 ? 3 : 2;
+}
+
 // T: warps per query.  1: a warp of its own for each query.  kTeamWarps (exact forms):
 // the block's warps search for one query (beam_search_team), for batches too small to
 // fill the device.
 template <int DM, int RK, int T>
-__global__ void __launch_bounds__(T == 1 ? 128 : 32 * T, T == 1 ? 4 : RK == 64 || RK == kRows4 ? 3 : 2) k_phase_a(DevView v, const float* __restrict__ Q, uint32_t nq,
+__global__ void __launch_bounds__(T == 1 ? 128 : 32 * T, phase_a_blocks(RK, T)) k_phase_a(DevView v, const float* __restrict__ Q, uint32_t nq,
                                                  const uint32_t* __restrict__ qm, const uint32_t* __restrict__ qef,
                                                  uint32_t efc, uint32_t vc, uint32_t mmax,
                                                  uint32_t* __restrict__ prox, uint32_t* __restrict__ nprox,
@@ -912,8 +925,8 @@ uint64_t search_batch(Index& ix, const SearchArgs& a) {
         } else {
             // one CTA per query (every query: the CTA path verifies a batch in one group)
             const size_t smem = bc_cta_smem(v.dim, counts_mode, mixed);
-            KCta kc = ix.wide ? pick_bc<uint64_t>(fusedsimd, counts_mode, mixed)
-                              : pick_bc<uint32_t>(fusedsimd, counts_mode, mixed);
+            KCta kc = ix.wide ? pick_bc<uint64_t>(fusedsimd, counts_mode, mixed, v)
+                              : pick_bc<uint32_t>(fusedsimd, counts_mode, mixed, v);
             CUDA_CHECK(cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             int per_sm = 1;
             CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kc, 256, smem));
@@ -1350,7 +1363,7 @@ void plan_create(SearchPlan& p, cudaStream_t s) {
     int per_sm = 1;
     CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfun, L.wpb * 32, L.smem_a));
     L.grid_a = (uint32_t)std::max<size_t>(1, std::min<size_t>(L.team ? nq : (nq + L.wpb - 1) / L.wpb, (size_t)nsm * std::max(per_sm, 1)));
-    KCta kc = ix.wide ? pick_bc<uint64_t>(L.fusedsimd, L.counts, L.mixed) : pick_bc<uint32_t>(L.fusedsimd, L.counts, L.mixed);
+    KCta kc = ix.wide ? pick_bc<uint64_t>(L.fusedsimd, L.counts, L.mixed, v) : pick_bc<uint32_t>(L.fusedsimd, L.counts, L.mixed, v);
     if (stream) {
         p.sb.reserve((uint32_t)nq, v.dim, nq * L.mstride, stream_max_chunks(nq * L.tmax, nq * L.mstride));
         stream_prepare(v, ix.wide, L.fusedsimd);
