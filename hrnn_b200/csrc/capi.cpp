@@ -198,7 +198,20 @@ hrnn_status hrnn_search_rknn_batch(hrnn_index* h, const float* q, size_t nq, con
         uint32_t* def = (uint32_t*)((char*)dkp + al(ib));
         uint64_t* doff = (uint64_t*)((char*)def + al(ib));
         uint64_t* dlab = (uint64_t*)((char*)doff + al(ob));
-        if (nq) {
+        // A small batch goes through pinned memory: its inputs in one copy, its offsets
+        // and first labels back with the search's own read-back.
+        const size_t in_b = al(qb) + 3 * al(ib);
+        const bool small = nq && in_b <= hrnn::kPinBytes && ob + 8 <= hrnn::kPinBytes / 2;
+        if (small && !ix.pin)
+            CUDA_CHECK(cudaMallocHost((void**)&ix.pin, sizeof(hrnn::SearchReads) + hrnn::kPinBytes));
+        char* pin = small ? ix.pin + sizeof(hrnn::SearchReads) : nullptr;
+        if (small) {
+            std::memcpy(pin, q, qb);
+            std::memcpy(pin + al(qb), m, ib);
+            std::memcpy(pin + al(qb) + al(ib), Kp, ib);
+            std::memcpy(pin + al(qb) + 2 * al(ib), ef, ib);
+            CUDA_CHECK(cudaMemcpyAsync(dq, pin, in_b, cudaMemcpyHostToDevice, s));
+        } else if (nq) {
             CUDA_CHECK(cudaMemcpyAsync(dq, q, qb, cudaMemcpyHostToDevice, s));
             CUDA_CHECK(cudaMemcpyAsync(dm, m, ib, cudaMemcpyHostToDevice, s));
             CUDA_CHECK(cudaMemcpyAsync(dkp, Kp, ib, cudaMemcpyHostToDevice, s));
@@ -209,11 +222,20 @@ hrnn_status hrnn_search_rknn_batch(hrnn_index* h, const float* q, size_t nq, con
             a.h_mmax = std::max(a.h_mmax, m[i]);
             a.h_efmax = std::max(a.h_efmax, std::max(ef[i], m[i]));
         }
+        if (small) {  // (the inputs are on the device by the time the answers come back)
+            a.h_stage = pin;
+            a.stage_labels = out_labels ? (hrnn::kPinBytes - ob) / 8 : 0;
+        }
         uint64_t total = hrnn::search_batch(ix, a);
-        CUDA_CHECK(cudaMemcpyAsync(out_offsets, doff, ob, cudaMemcpyDeviceToHost, s));
-        if (total <= cap && total && out_labels)
-            CUDA_CHECK(cudaMemcpyAsync(out_labels, dlab, total * 8, cudaMemcpyDeviceToHost, s));
-        CUDA_CHECK(cudaStreamSynchronize(s));
+        if (small && (total <= a.stage_labels || total > cap || !out_labels)) {
+            std::memcpy(out_offsets, pin, ob);
+            if (total <= cap && total && out_labels) std::memcpy(out_labels, pin + ob, total * 8);
+        } else {
+            CUDA_CHECK(cudaMemcpyAsync(out_offsets, doff, ob, cudaMemcpyDeviceToHost, s));
+            if (total <= cap && total && out_labels)
+                CUDA_CHECK(cudaMemcpyAsync(out_labels, dlab, total * 8, cudaMemcpyDeviceToHost, s));
+            CUDA_CHECK(cudaStreamSynchronize(s));
+        }
         if (total > cap) hrnn::fail(HRNN_ERR_CAPACITY, "searchRknn: output capacity too small");
     });
 }

@@ -19,6 +19,9 @@ Index::Index() = default;
 Index::~Index() {
     for (auto& e : aux_ev)
         if (e) cudaEventDestroy(e);
+    for (auto& e : phase_ev)
+        if (e) cudaEventDestroy(e);
+    if (pin) cudaFreeHost(pin);
     if (aux) cudaStreamDestroy(aux);
     if (stream) cudaStreamDestroy(stream);
 }

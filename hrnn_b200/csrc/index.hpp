@@ -54,6 +54,14 @@ struct SearchCounters {
     unsigned long long n_lowp, n_fp32, n_fp64, n_flip, overflow;
 };
 
+// Numbers a batch call reads back from the device.
+struct SearchReads {
+    uint64_t postings, total;
+    uint32_t n_overflow, pad;
+    SearchCounters counters;
+};
+constexpr size_t kPinBytes = 64 << 10;
+
 // Device mutable reverse lists (rknng_mutable.cu): element i's owners in
 // ent[off[i] .. off[i] + len[i]), cap[i] slots.
 struct MutableLists {
@@ -151,6 +159,10 @@ struct Index {
     // beside the verification of the queries it does not concern
     cudaStream_t aux = nullptr;
     cudaEvent_t aux_ev[2] = {nullptr, nullptr};
+    cudaEvent_t phase_ev[4] = {nullptr, nullptr, nullptr, nullptr};  // a batch call's phases
+    // pinned: what a batch call reads back (SearchReads), then kPinBytes for a small
+    // batch's inputs and answers
+    char* pin = nullptr;
     DevMem io;           // host-buffer entry points stage their inputs/outputs here
     DevMem counters;     // SearchCounters
     DevMem kcol;         // f32 [n]: kdist(p, k-1) of the current search call
@@ -207,6 +219,10 @@ struct SearchArgs {
     // the batch's largest m and max(ef, m) when the caller knows them (host
     // inputs); 0: read back from d_m / d_ef
     uint32_t h_mmax = 0, h_efmax = 0;
+    // pinned place for the offsets and the first stage_labels labels (null: not wanted),
+    // filled when the call returns
+    char* h_stage = nullptr;
+    size_t stage_labels = 0;
 };
 uint64_t search_batch(Index& ix, const SearchArgs& a);  // returns total results
 void kdist_column(Index& ix, uint32_t k, float* host_out);  // kdist(p, k-1) of every element

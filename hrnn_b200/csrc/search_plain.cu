@@ -491,12 +491,14 @@ __global__ void k_plan_inputs(const uint32_t* __restrict__ m_in, const uint32_t*
     ef_out[i] = min(ef, ef_max);
 }
 
-// k_pack_results when the total (out_off[nq]) fits the caller's capacity.
+// k_pack_results when the total (out_off[nq]) fits the caller's capacity and no query
+// waits for the overflow pass (*n_overflow; may be null).
 __global__ void k_pack_results_capped(uint32_t nq, const uint64_t* __restrict__ res_off,
                                       const uint32_t* __restrict__ res_count, const uint64_t* __restrict__ out_off,
-                                      const uint64_t* __restrict__ resbuf, uint64_t* __restrict__ out, size_t cap) {
+                                      const uint64_t* __restrict__ resbuf, uint64_t* __restrict__ out, size_t cap,
+                                      const uint32_t* __restrict__ n_overflow) {
     const uint32_t qi = blockIdx.x;
-    if (qi >= nq || out_off[nq] > cap) return;
+    if (qi >= nq || out_off[nq] > cap || (n_overflow && *n_overflow)) return;
     const uint32_t c = res_count[qi];
     for (uint32_t i = threadIdx.x; i < c; i += blockDim.x) out[out_off[qi] + i] = resbuf[res_off[qi] + i];
 }
@@ -628,14 +630,16 @@ uint64_t search_batch(Index& ix, const SearchArgs& a) {
     if (ix.serve_mode && (a.k == 0 || a.k > ix.max_k_serve))
         fail(HRNN_ERR_ARG, "searchRknn: k must be in [1, max_k_serve] in serve mode");
     ix.sync_upper_to_device();
-    cudaEvent_t ev[4];
-    for (auto& e : ev) CUDA_CHECK(cudaEventCreate(&e));
+    cudaEvent_t* const ev = ix.phase_ev;
+    for (int i = 0; i < 4; ++i)
+        if (!ev[i]) CUDA_CHECK(cudaEventCreate(&ev[i]));
+    if (!ix.pin) CUDA_CHECK(cudaMallocHost((void**)&ix.pin, sizeof(SearchReads) + kPinBytes));
+    SearchReads& rd = *reinterpret_cast<SearchReads*>(ix.pin);
     CUDA_CHECK(cudaMemsetAsync(ix.counters.p, 0, sizeof(SearchCounters), s));
     const unsigned long long launches0 = launch_counter().load();
     if (nq == 0) {
         CUDA_CHECK(cudaMemsetAsync(a.d_out_offsets, 0, 8, s));
         CUDA_CHECK(cudaStreamSynchronize(s));
-        for (auto& e : ev) cudaEventDestroy(e);
         ix.last_stats = hrnn_search_stats{};
         return 0;
     }
@@ -882,10 +886,58 @@ uint64_t search_batch(Index& ix, const SearchArgs& a) {
         }
     }
     CUDA_CHECK(cudaEventRecord(ev[1], s));
+    const uint32_t kidx = (uint32_t)(a.k - 1);
+    uint32_t* const d_nov = d_next + 1;  // spare counters after d_next, zeroed with d_rcount
+    uint32_t* ovl = nullptr;
+    // Queries whose shared-memory table or accepted list overflowed: the global-memory
+    // warp kernel, with a table sized for their posting count.
+    auto run_overflow = [&](uint32_t nov, const uint64_t* d_tot, const uint64_t* d_off, uint64_t* rbuf) {
+        std::vector<uint32_t> hov(nov);
+        std::vector<uint64_t> htot(nq);
+        CUDA_CHECK(cudaMemcpyAsync(hov.data(), ovl, nov * 4, cudaMemcpyDeviceToHost, s));
+        CUDA_CHECK(cudaMemcpyAsync(htot.data(), d_tot, nq * 8, cudaMemcpyDeviceToHost, s));
+        CUDA_CHECK(cudaStreamSynchronize(s));
+        uint64_t tmax = 1;
+        for (uint32_t qi : hov) tmax = std::max(tmax, htot[qi]);
+        DevMem& hkey = ix.scratch[5];
+        DevMem& hcnt = ix.scratch[6];
+        uint32_t hcap = 64;
+        while (hcap < 2 * tmax) hcap <<= 1;
+        size_t per_slot = (size_t)hcap * 8 + tmax * 4;
+        size_t slots = std::max<size_t>(1, std::min<size_t>((size_t)nsm * 8 * 4, (size_t)(4ull << 30) / per_slot));
+        slots = std::min<size_t>(slots, ((size_t)nov + 3) / 4 * 4);
+        slots = (slots + 3) / 4 * 4;
+        size_t need_h = slots * (size_t)hcap * 4;
+        if (hkey.bytes < need_h) {
+            hkey.alloc(need_h);
+            hcnt.alloc(need_h);
+            CUDA_CHECK(cudaMemsetAsync(hkey.p, 0xFF, need_h, s));
+            CUDA_CHECK(cudaMemsetAsync(hcnt.p, 0, need_h, s));
+        }
+        DevMem& lp = ix.scratch[4];
+        lp.ensure(slots * tmax * 4 + 64);
+        uint32_t* d_next2 = d_next + 2;
+        CUDA_CHECK(cudaMemsetAsync(d_next2, 0, 4, s));
+        size_t smem_w = 4 * (v.dim * 4 + 16);
+        void (*kern)(DevView, const float*, uint32_t, uint32_t, const uint32_t*, const uint32_t*, const uint32_t*,
+                     const uint64_t*, float, uint32_t, uint32_t, uint32_t*, uint32_t*, uint32_t*, size_t,
+                     uint64_t*, uint32_t*, uint32_t*, const uint32_t*, SearchCounters*, const uint32_t*,
+                     uint32_t*);
+        if (ix.wide) kern = fusedsimd ? k_phase_bc<uint64_t, true> : k_phase_bc<uint64_t, false>;
+        else kern = fusedsimd ? k_phase_bc<uint32_t, true> : k_phase_bc<uint32_t, false>;
+        kern<<<(unsigned)(slots / 4), 128, smem_w, s>>>(v, a.d_q, nov, mmax, prox.as<uint32_t>(),
+                                                        nprox.as<uint32_t>(), plen.as<uint32_t>(), d_off,
+                                                        a.threshold, kidx, hcap, hkey.as<uint32_t>(),
+                                                        hcnt.as<uint32_t>(), lp.as<uint32_t>(), (size_t)tmax,
+                                                        rbuf, d_rcount, d_next2, ovl, ctr, nullptr, nullptr);
+        CUDA_LAUNCH_CHECK();
+    };
     // Phase B (posting counts, staging) and C (verification) of the queries with
-    // g[q] == want (all of them for g null), staged in `resm` at offsets d_off.
+    // g[q] == want (all of them for g null), staged in `resm` at offsets d_off.  The one
+    // wait in it is for the posting total, which sizes the staging; with `later` the
+    // overflow count is left for the caller to read with the total.
     auto run_bc = [&](const uint8_t* g, uint8_t want, uint64_t* d_tot, uint64_t* d_off, DevMem& resm,
-                      bool first) -> uint64_t* {
+                      bool first, bool later) -> uint64_t* {
         {
             size_t tot = nq * mmax;
             auto kern = ix.wide ? k_phase_b_count<uint64_t> : k_phase_b_count<uint32_t>;
@@ -895,26 +947,20 @@ uint64_t search_batch(Index& ix, const SearchArgs& a) {
             CUDA_LAUNCH_CHECK();
         }
         exclusive_scan_u64(d_tot, d_off, nq + 1, s, tmp);
-        std::vector<uint64_t> htot(nq);
-        uint64_t sum_total = 0;
-        CUDA_CHECK(cudaMemcpyAsync(htot.data(), d_tot, nq * 8, cudaMemcpyDeviceToHost, s));
-        CUDA_CHECK(cudaMemcpyAsync(&sum_total, d_off + nq, 8, cudaMemcpyDeviceToHost, s));
-        CUDA_CHECK(cudaStreamSynchronize(s));
-        DevMem& hkey = ix.scratch[5];
-        DevMem& hcnt = ix.scratch[6];
-        const size_t res_bytes = std::max<uint64_t>(sum_total, 1) * 8;
-        resm.ensure(res_bytes + (nq + 1) * 4 + 256);
-        uint64_t* rbuf = resm.as<uint64_t>();
-        uint32_t* ovl = (uint32_t*)(resm.as<char>() + ((res_bytes + 255) & ~(size_t)255));
-        uint32_t* d_nov = d_next + 1;  // spare counters after d_next, zeroed with d_rcount
-        if (first) CUDA_CHECK(cudaEventRecord(ev[2], s));
-        // Per-call column of kdist(p, k-1) (hrnn.h:286-293), then the verification.
-        const uint32_t kidx = (uint32_t)(a.k - 1);
+        CUDA_CHECK(cudaMemcpyAsync(&rd.postings, d_off + nq, 8, cudaMemcpyDeviceToHost, s));
+        // Per-call column of kdist(p, k-1) (hrnn.h:286-293), for the verification.
         if (first) {
+            CUDA_CHECK(cudaEventRecord(ev[2], s));
             ix.kcol.ensure((size_t)std::max<size_t>(ix.cur, 1) * 4);
             k_kdist_column<<<(unsigned)((ix.cur + 255) / 256), 256, 0, s>>>(v, kidx, ix.kcol.as<float>());
             CUDA_LAUNCH_CHECK();
         }
+        CUDA_CHECK(cudaStreamSynchronize(s));
+        const uint64_t sum_total = rd.postings;
+        const size_t res_bytes = std::max<uint64_t>(sum_total, 1) * 8;
+        resm.ensure(res_bytes + (nq + 1) * 4 + 256);
+        uint64_t* rbuf = resm.as<uint64_t>();
+        ovl = (uint32_t*)(resm.as<char>() + ((res_bytes + 255) & ~(size_t)255));
         if (stream_bc) {
             // INT8 form: postings verified as they are read, in chunks spread over
             // persistent warps
@@ -936,50 +982,14 @@ uint64_t search_batch(Index& ix, const SearchArgs& a) {
                                        rbuf, d_rcount, d_next, ovl, d_nov, ctr);
             CUDA_LAUNCH_CHECK();
         }
-        // Queries whose shared-memory table or accepted list overflowed: the
-        // global-memory warp kernel, with a table sized for their posting count.
-        uint32_t nov = 0;
-        CUDA_CHECK(cudaMemcpyAsync(&nov, d_nov, 4, cudaMemcpyDeviceToHost, s));
-        CUDA_CHECK(cudaStreamSynchronize(s));
-        if (nov) {
-            std::vector<uint32_t> hov(nov);
-            CUDA_CHECK(cudaMemcpy(hov.data(), ovl, nov * 4, cudaMemcpyDeviceToHost));
-            uint64_t tmax = 1;
-            for (uint32_t qi : hov) tmax = std::max(tmax, htot[qi]);
-            uint32_t hcap = 64;
-            while (hcap < 2 * tmax) hcap <<= 1;
-            size_t per_slot = (size_t)hcap * 8 + tmax * 4;
-            size_t slots = std::max<size_t>(1, std::min<size_t>((size_t)nsm * 8 * 4, (size_t)(4ull << 30) / per_slot));
-            slots = std::min<size_t>(slots, ((size_t)nov + 3) / 4 * 4);
-            slots = (slots + 3) / 4 * 4;
-            size_t need_h = slots * (size_t)hcap * 4;
-            if (hkey.bytes < need_h) {
-                hkey.alloc(need_h);
-                hcnt.alloc(need_h);
-                CUDA_CHECK(cudaMemsetAsync(hkey.p, 0xFF, need_h, s));
-                CUDA_CHECK(cudaMemsetAsync(hcnt.p, 0, need_h, s));
-            }
-            DevMem& lp = ix.scratch[4];
-            lp.ensure(slots * tmax * 4 + 64);
-            uint32_t* d_next2 = d_next + 2;
-            CUDA_CHECK(cudaMemsetAsync(d_next2, 0, 4, s));
-            size_t smem_w = 4 * (v.dim * 4 + 16);
-            void (*kern)(DevView, const float*, uint32_t, uint32_t, const uint32_t*, const uint32_t*, const uint32_t*,
-                         const uint64_t*, float, uint32_t, uint32_t, uint32_t*, uint32_t*, uint32_t*, size_t,
-                         uint64_t*, uint32_t*, uint32_t*, const uint32_t*, SearchCounters*, const uint32_t*,
-                         uint32_t*);
-            if (ix.wide) kern = fusedsimd ? k_phase_bc<uint64_t, true> : k_phase_bc<uint64_t, false>;
-            else kern = fusedsimd ? k_phase_bc<uint32_t, true> : k_phase_bc<uint32_t, false>;
-            kern<<<(unsigned)(slots / 4), 128, smem_w, s>>>(v, a.d_q, nov, mmax, prox.as<uint32_t>(),
-                                                            nprox.as<uint32_t>(), plen.as<uint32_t>(), d_off,
-                                                            a.threshold, kidx, hcap, hkey.as<uint32_t>(),
-                                                            hcnt.as<uint32_t>(), lp.as<uint32_t>(), (size_t)tmax,
-                                                            rbuf, d_rcount, d_next2, ovl, ctr, nullptr, nullptr);
-            CUDA_LAUNCH_CHECK();
+        if (!later) {
+            CUDA_CHECK(cudaMemcpyAsync(&rd.n_overflow, d_nov, 4, cudaMemcpyDeviceToHost, s));
+            CUDA_CHECK(cudaStreamSynchronize(s));
+            if (rd.n_overflow) run_overflow(rd.n_overflow, d_tot, d_off, rbuf);
         }
         return rbuf;
     };
-    uint64_t* resbuf = run_bc(split ? grp : nullptr, 0, d_total, d_resoff, ix.scratch[7], true);
+    uint64_t* resbuf = run_bc(split ? grp : nullptr, 0, d_total, d_resoff, ix.scratch[7], true, !split);
     uint64_t *resbuf2 = nullptr, *d_total2 = nullptr, *d_resoff2 = nullptr;
     if (split) {
         // group 1 once its second search is done
@@ -990,26 +1000,51 @@ uint64_t search_batch(Index& ix, const SearchArgs& a) {
         CUDA_CHECK(cudaStreamWaitEvent(s, ix.aux_ev[1], 0));
         CUDA_CHECK(cudaMemsetAsync(d_total2, 0, (nq + 1) * 8, s));
         CUDA_CHECK(cudaMemsetAsync(d_next, 0, 12, s));  // the verification's counters of group 0
-        resbuf2 = run_bc(grp, 1, d_total2, d_resoff2, ix.scratch[8], false);
+        resbuf2 = run_bc(grp, 1, d_total2, d_resoff2, ix.scratch[8], false, false);
     }
-    exclusive_scan_u32_to_u64(d_rcount, a.d_out_offsets, nq + 1, s, tmp);
-    uint64_t total = 0;
-    CUDA_CHECK(cudaMemcpyAsync(&total, a.d_out_offsets + nq, 8, cudaMemcpyDeviceToHost, s));
-    CUDA_CHECK(cudaStreamSynchronize(s));
-    if (total <= a.cap && total > 0) {
-        k_pack_results<<<(unsigned)nq, 128, 0, s>>>((uint32_t)nq, d_resoff, d_rcount, a.d_out_offsets, resbuf,
-                                                     a.d_out_labels, split ? grp : nullptr, 0);
+    // Offsets, labels (where they fit the capacity) and everything the host reads, with
+    // one wait; a batch with queries for the overflow pass goes round once more.
+    const size_t stage = a.h_stage ? std::min(a.cap, a.stage_labels) : 0;
+    for (bool again = true; again;) {
+        exclusive_scan_u32_to_u64(d_rcount, a.d_out_offsets, nq + 1, s, tmp);
+        k_pack_results_capped<<<(unsigned)nq, 128, 0, s>>>((uint32_t)nq, d_resoff, d_rcount, a.d_out_offsets, resbuf,
+                                                            a.d_out_labels, split ? 0 : a.cap, d_nov);
         CUDA_LAUNCH_CHECK();
-        if (split) {
-            k_pack_results<<<(unsigned)nq, 128, 0, s>>>((uint32_t)nq, d_resoff2, d_rcount, a.d_out_offsets, resbuf2,
-                                                         a.d_out_labels, grp, 1);
-            CUDA_LAUNCH_CHECK();
+        CUDA_CHECK(cudaEventRecord(ev[3], s));
+        CUDA_CHECK(cudaMemcpyAsync(&rd.total, a.d_out_offsets + nq, 8, cudaMemcpyDeviceToHost, s));
+        CUDA_CHECK(cudaMemcpyAsync(&rd.n_overflow, d_nov, 4, cudaMemcpyDeviceToHost, s));
+        CUDA_CHECK(cudaMemcpyAsync(&rd.counters, ix.counters.p, sizeof(SearchCounters), cudaMemcpyDeviceToHost, s));
+        if (a.h_stage && !split) {
+            CUDA_CHECK(cudaMemcpyAsync(a.h_stage, a.d_out_offsets, (nq + 1) * 8, cudaMemcpyDeviceToHost, s));
+            if (stage)
+                CUDA_CHECK(cudaMemcpyAsync(a.h_stage + (nq + 1) * 8, a.d_out_labels, stage * 8,
+                                           cudaMemcpyDeviceToHost, s));
+        }
+        CUDA_CHECK(cudaStreamSynchronize(s));
+        again = !split && rd.n_overflow;
+        if (again) {
+            run_overflow(rd.n_overflow, d_total, d_resoff, resbuf);
+            CUDA_CHECK(cudaMemsetAsync(d_nov, 0, 4, s));
         }
     }
-    CUDA_CHECK(cudaEventRecord(ev[3], s));
-    CUDA_CHECK(cudaStreamSynchronize(s));
-    SearchCounters hc{};
-    CUDA_CHECK(cudaMemcpy(&hc, ix.counters.p, sizeof(hc), cudaMemcpyDeviceToHost));
+    const uint64_t total = rd.total;
+    if (split && total <= a.cap && total > 0) {
+        k_pack_results<<<(unsigned)nq, 128, 0, s>>>((uint32_t)nq, d_resoff, d_rcount, a.d_out_offsets, resbuf,
+                                                     a.d_out_labels, grp, 0);
+        CUDA_LAUNCH_CHECK();
+        k_pack_results<<<(unsigned)nq, 128, 0, s>>>((uint32_t)nq, d_resoff2, d_rcount, a.d_out_offsets, resbuf2,
+                                                     a.d_out_labels, grp, 1);
+        CUDA_LAUNCH_CHECK();
+        CUDA_CHECK(cudaEventRecord(ev[3], s));
+        CUDA_CHECK(cudaStreamSynchronize(s));
+    }
+    if (split && a.h_stage) {  // two groups: the answers are complete only now
+        CUDA_CHECK(cudaMemcpyAsync(a.h_stage, a.d_out_offsets, (nq + 1) * 8, cudaMemcpyDeviceToHost, s));
+        if (stage)
+            CUDA_CHECK(cudaMemcpyAsync(a.h_stage + (nq + 1) * 8, a.d_out_labels, stage * 8, cudaMemcpyDeviceToHost, s));
+        CUDA_CHECK(cudaStreamSynchronize(s));
+    }
+    const SearchCounters hc = rd.counters;
     if (learned) {
         CUDA_CHECK(cudaMemcpy(ix.budget->n_level, ix.budget->decided.as<char>() + 8, 24, cudaMemcpyDeviceToHost));
         ix.budget->mlp.check_tc();
@@ -1039,7 +1074,6 @@ uint64_t search_batch(Index& ix, const SearchArgs& a) {
     st.phase_b_ms = t12;
     st.phase_c_ms = t23;
     ix.last_stats = st;
-    for (auto& e : ev) cudaEventDestroy(e);
     return total;
 }
 
@@ -1476,7 +1510,7 @@ void plan_create(SearchPlan& p, cudaStream_t s) {
     }
     exclusive_scan_u32_to_u64(d_rcount, p.d_out_off, nq + 1, s, p.tmp);
     k_pack_results_capped<<<(unsigned)nq, 128, 0, s>>>((uint32_t)nq, pack_off, d_rcount, p.d_out_off, resbuf,
-                                                        p.d_out_lab, p.cap);
+                                                        p.d_out_lab, p.cap, nullptr);
     } catch (...) {
         cudaGraph_t g = nullptr;
         cudaStreamEndCapture(s, &g);  // leave the stream usable
