@@ -397,17 +397,6 @@ __device__ __forceinline__ void load_row(const DevView& v, uint32_t c, int level
     w1 = (lane == 0 && W > 32) ? __ldg(row + 32) : 0u;
 }
 
-// First index in td[0..n) with td[i] > x.
-__device__ __forceinline__ uint32_t upper_bound(const float* td, uint32_t n, float x) {
-    uint32_t lo = 0, hi = n;
-    while (lo < hi) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (td[mid] > x) hi = mid;
-        else lo = mid + 1;
-    }
-    return lo;
-}
-
 // ---------------------------------------------------------------------------
 // BF16 rows (mixed-precision search): vec_bf16[n][dim] holds round-to-nearest
 // copies of the FP32 rows.  These distances rank candidates only; every

@@ -305,16 +305,17 @@ __global__ void k_sample_rev(uint32_t n, uint32_t R, uint32_t cap, const uint64_
 // ---- phase 2: join -----------------------------------------------------------
 
 // One block (16 warps) per node of the chunk at a time: exact FP32 distances of
-// all sample pairs.  The node's rows are staged in shared memory (stride dim + 4
-// floats: 16-byte aligned and free of bank conflicts for float4 reads).  Work
+// all sample pairs.  The node's rows are staged in shared memory (an odd number of
+// 16-byte units apart: free of bank conflicts for float4 reads).  Work
 // unit: kJR rows i0 .. i0 + 3 (a row tile of the new list) x one column j > i0;
 // a tile's columns run from i0 + 1 to the last row, and the units of all tiles
 // are numbered consecutively, so a warp takes 32 consecutive units (lane = unit)
 // and no lane computes a pair below the diagonal or past the last row.  The row
 // vectors are mostly read by the whole warp at one address (broadcast) and the
 // lane's column vector once for all kJR pairs, so a 16-byte shared-memory read
-// feeds 4 kJR elementwise steps.  Each pair keeps the reference's 16
-// accumulators (element e into accumulator e mod 16, then summed left to right),
+// feeds 4 kJR elementwise steps.  Each pair keeps the reference's L
+// accumulators (element e into accumulator e mod L, then summed left to right; L =
+// 16, or 4 for dims that are multiples of 4 but not of 16),
 // so the tiling leaves every distance bit-identical.
 //
 // NBUF 1 (256 threads, two blocks per SM): one stage per block, the default.
@@ -334,8 +335,11 @@ __device__ __forceinline__ uint32_t join_units_before(uint32_t a, uint32_t tot) 
     return a * (tot - 1) - (kJR / 2) * a * (a - 1);
 }
 
+// Floats between staged rows.
+__host__ __device__ inline uint32_t join_row_floats(uint32_t dim) { return 4 * ((dim >> 2) | 1u); }
+
 __host__ __device__ inline size_t join_stage_floats(uint32_t dim, uint32_t cap) {
-    return (size_t)(2 * cap + kJR) * (dim + 4);
+    return (size_t)(2 * cap + kJR) * join_row_floats(dim);
 }
 
 __host__ __device__ inline size_t join_smem_bytes(uint32_t dim, uint32_t cap, int nbuf) {
@@ -347,7 +351,7 @@ constexpr int join_threads() {
     return NBUF == 2 ? 512 : 256;
 }
 
-template <bool FUSED, int NBUF>
+template <bool FUSED, int NBUF, int L>
 __global__ void __launch_bounds__(join_threads<NBUF>(), NBUF == 2 ? 1 : 2) k_join(const float* __restrict__ vec, uint32_t dim, uint32_t node0,
                                                  uint32_t node1, uint32_t cap, const uint32_t* __restrict__ newl,
                                                  const uint32_t* __restrict__ newc, const uint32_t* __restrict__ oldl,
@@ -355,7 +359,7 @@ __global__ void __launch_bounds__(join_threads<NBUF>(), NBUF == 2 ? 1 : 2) k_joi
                                                  Prop* __restrict__ prop, unsigned long long* __restrict__ pcount,
                                                  unsigned long long pcap, unsigned long long* __restrict__ njoin) {
     extern __shared__ __align__(16) float sm[];
-    const uint32_t SP = dim + 4;
+    const uint32_t SP = join_row_floats(dim);
     const size_t stage = join_stage_floats(dim, cap);
     // stage b: rows at sm + b stage, then (after all stages) ids and thresholds
     uint32_t* const ids0 = (uint32_t*)(sm + NBUF * stage);
@@ -427,18 +431,18 @@ __global__ void __launch_bounds__(join_threads<NBUF>(), NBUF == 2 ? 1 : 2) k_joi
             }
             const uint32_t i0 = lo * kJR;
             const uint32_t j = i0 + 1 + (fc - join_units_before(lo, tot));
-            float acc[kJR][16];
+            float acc[kJR][L];
 #pragma unroll
             for (int r = 0; r < kJR; ++r)
 #pragma unroll
-                for (int l = 0; l < 16; ++l) acc[r][l] = 0.f;
+                for (int l = 0; l < L; ++l) acc[r][l] = 0.f;
             // rows past the staged ones (i0 + r >= tot) read the spare rows at the
             // end of the stage; their sums are never used
             const float4* xb = reinterpret_cast<const float4*>(R + (size_t)j * SP);
             const float4* xa = reinterpret_cast<const float4*>(R + (size_t)i0 * SP);
-            for (uint32_t e4 = 0; e4 < d4; e4 += 4) {
+            for (uint32_t e4 = 0; e4 < d4; e4 += L / 4) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
+                for (int c = 0; c < L / 4; ++c) {
                     const float4 bb = xb[e4 + c];
 #pragma unroll
                     for (int r = 0; r < kJR; ++r) {
@@ -458,7 +462,7 @@ __global__ void __launch_bounds__(join_threads<NBUF>(), NBUF == 2 ? 1 : 2) k_joi
             for (int r = 0; r < kJR; ++r) {
                 float dv = acc[r][0];
 #pragma unroll
-                for (int l = 1; l < 16; ++l) dv = __fadd_rn(dv, acc[r][l]);
+                for (int l = 1; l < L; ++l) dv = __fadd_rn(dv, acc[r][l]);
                 dd[r] = dv;
                 const uint32_t i = i0 + r;
                 if (live && i < nn && j > i && ids[i] != bj) {
@@ -566,7 +570,8 @@ __global__ void __launch_bounds__(join_threads<NBUF>(), NBUF == 2 ? 1 : 2) k_joi
     atomicAdd(njoin, local_pairs);
 }
 
-// Generic-dim fallback (dims not a multiple of 16, or 8/4-lane orders): one thread
+// Generic-dim fallback (dims not a multiple of 4, multiples of 16 under the 8/4-lane
+// orders, and samples that do not fit in shared memory): one thread
 // per pair reading global memory.
 __global__ void k_join_generic(const float* __restrict__ vec, uint32_t dim, int lanes, int fused, uint32_t node0,
                                uint32_t node1, uint32_t cap, const uint32_t* __restrict__ newl,
@@ -1440,9 +1445,13 @@ void refine_knng(Index& ix, int iters, int sample) {
     uint32_t* d_nextt = (uint32_t*)(ctr.as<unsigned long long>() + 3);  // merge work counter
     unsigned long long* d_pcount = ctr.as<unsigned long long>();  // proposal slots of a chunk
     unsigned long long* d_nprop = ctr.as<unsigned long long>() + 5;  // proposals of the iteration
-    const bool fast = ix.order.lanes == 16 && ix.dim % 16 == 0;
+    const bool rows16 = ix.order.lanes == 16 && ix.dim % 16 == 0;
+    // (dims that are multiples of 4 only: with one thread per pair the joins of a 5k x
+    // 100 build's five iterations took 6.9 ms, staged in shared memory 0.74)
+    const bool rows4 = ix.dim % 4 == 0 && ix.dim % 16 != 0 && join_smem_bytes((uint32_t)ix.dim, cap, 1) <= 227 * 1024;
+    const bool fast = rows16 || rows4;
     // Tensor-core screened join where the dims and sample sizes allow it.
-    const bool tcj = fast && ix.join_mode != kJoinExact && join_tc_supported((uint32_t)ix.dim, cap);
+    const bool tcj = rows16 && ix.join_mode != kJoinExact && join_tc_supported((uint32_t)ix.dim, cap);
     JoinTcCounters* d_jc = reinterpret_cast<JoinTcCounters*>(ctr.as<char>() + 64);
     // The exact join's two forms: two stages (the next node's rows copied during
     // the current node's pairs) for iterations with many pairs per node, where two
@@ -1460,8 +1469,8 @@ void refine_knng(Index& ix, int iters, int sample) {
     if (const char* e = std::getenv("HRNN_JOIN2_MIN_PAIRS")) join2_min_pairs = std::strtod(e, nullptr);
     const size_t join_smem1 = join_smem_bytes((uint32_t)ix.dim, cap, 1);
     const size_t join_smem2 = join_smem_bytes((uint32_t)ix.dim, cap, 2);
-    auto kj1 = jf ? k_join<true, 1> : k_join<false, 1>;
-    auto kj2 = jf ? k_join<true, 2> : k_join<false, 2>;
+    auto kj1 = rows4 ? (jf ? k_join<true, 1, 4> : k_join<false, 1, 4>) : (jf ? k_join<true, 1, 16> : k_join<false, 1, 16>);
+    auto kj2 = rows4 ? (jf ? k_join<true, 2, 4> : k_join<false, 2, 4>) : (jf ? k_join<true, 2, 16> : k_join<false, 2, 16>);
     unsigned join_grid1 = (unsigned)nsm, join_grid2 = (unsigned)nsm;
     if (fast) {
         if (join_smem1 > 227 * 1024) fail(HRNN_ERR_ARG, "refineKNNG: sample size too large for dim");
