@@ -7,7 +7,8 @@
 //   2. exclusive scan -> u64 offsets, exactly the reference's rknng_offsets_
 //   3. scatter (owner << rank_bits) | rank with per-target atomic cursors
 //   4. sort every segment by (rank, owner): one warp per segment of <= 1024
-//      entries (bitonic network in shared memory), one block per larger segment.
+//      entries (bitonic network in registers), one block per larger segment
+//      (steps 3 and 4: csr_kernels.cuh).
 // Step 4 makes the result independent of the scatter order: each segment holds
 // exactly the reference's entries, grouped by rank like the reference's, with ties
 // in owner order (the reference's std::sort leaves ties in an unspecified order;

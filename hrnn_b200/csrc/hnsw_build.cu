@@ -3,8 +3,9 @@
 // of hrnn.h:1479-1501.
 //
 // Points are inserted in batches that grow with the index (1/24 of the current
-// size, at most 16384 points).  For every point of a batch one warp runs, against
-// the graph as it was at the start of the batch:
+// size, at most 16384 points) and are all enqueued without a wait.  For every point of
+// a batch one warp, or a team of warps while batches are small, runs against the
+// graph as it was at the start of the batch:
 //   - the greedy descent from the entry point down to the point's level + 1;
 //   - per level l <= min(level, maxlevel): the ef_construction beam search of
 //     that layer (beam.cuh), the KNN-graph seed at level 0 (the beam, ascending,
@@ -12,8 +13,9 @@
 //     getNeighborsByHeuristic2 (hrnn.h:619-659) choosing at most M links, written
 //     in the reference's order (farthest first, hrnn.h:695-699) -- the nearest
 //     link is the entry point of the next level (hrnn.h:700);
-//   - one reverse-link request (target list, new point, distance) per link.
-// Then k_link_update applies all requests of the batch, one warp per target
+//   - one link back (target list, new point, distance) per link, into the target
+//     list's slots.
+// Then k_link_update applies all links back of the batch, one warp per target
 // list: new points are appended while the list has room, otherwise the union of
 // the list and the new points is pruned with the same heuristic to maxM0 (level
 // 0) or maxM links (mutuallyConnectNewElement, hrnn.h:729-797).

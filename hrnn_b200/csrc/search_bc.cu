@@ -7,8 +7,8 @@
 //      posting is re-read P times; postings are 4 bytes, candidates 512).
 //   C: every distinct owner whose count reaches the threshold (hrnn.h:2043-2052)
 //      is verified in exact FP32, d(q,p) <= kdist(p, k-1) (hrnn.h:2058-2069):
-//      the warps sweep the table, compact candidates with a ballot and verify four
-//      per warp step (two per half-warp, loads issued together).  kdist(p, k-1) is
+//      the warps sweep the table, compact candidates with a ballot and verify up to
+//      32 at a time, four lanes per row.  kdist(p, k-1) is
 //      read from kcol, a per-call column of the KNN-slot radius (FLT_MAX when the
 //      list is shorter than k, hrnn.h:290-291) that stays resident in L2.
 //   Accepted ids of one range are sorted (bitonic, shared memory) and appended as

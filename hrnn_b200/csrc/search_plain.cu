@@ -1,7 +1,7 @@
 // Batched RkNN search, plain form: answers bit-identical to the reference's
 // searchRknn (hrnn.h:1966-2071) on the same index.
 //
-// Kernel A (one warp per query): greedy descent over the upper layers
+// Kernel A (one warp per query, or a team of warps for few queries): greedy descent over the upper layers
 // (hrnn.h:1992-2013) and the best-first base-layer search searchBaseLayerST
 // (hrnn.h:484-616) with ef = max(ef_search, m), trimmed to the m nearest proxies
 // (hrnn.h:2016-2019).  The beam formulation and its equivalence argument are in
@@ -10,7 +10,8 @@
 // Kernel B: length of each proxy's reverse-list prefix with rank < K' (binary
 // search: segments are sorted by rank), and the per-query total.
 //
-// Kernel C (warp per query): phase B posting scan into a per-warp open-address
+// Kernel C (one CTA per query, search_bc.cu; here the overflow pass, one warp per query
+// with tables in global memory): phase B posting scan into a per-warp open-address
 // table (the reference's score_buf counts), threshold filter and reset, exact
 // FP32 verification against the stored kNN radius, results in ascending
 // internal-id order (hrnn.h:2021-2070).
