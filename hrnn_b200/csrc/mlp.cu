@@ -22,6 +22,7 @@
 
 #include "index.hpp"
 #include "mlp.hpp"
+#include "mlp_ranges.hpp"
 
 namespace hrnn {
 
@@ -29,7 +30,7 @@ namespace {
 
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
-constexpr int kTile = 64, kTileK = 16;  // GEMM tiles; 256 threads, 4 x 4 outputs each
+constexpr int kTile = 64;  // GEMM tiles (kTileK deep); 256 threads, 4 x 4 outputs each
 
 // Z[M x 2] = A[M x 256] W^T + b (W [2 x 256]): a thread sums one row's both outputs over
 // k in order.  Rows are staged 32 columns at a time so the loads stay coalesced.
@@ -234,18 +235,6 @@ __global__ void __launch_bounds__(256) k_weight_grad3(const float* __restrict__ 
     if (t < kMlpOut) p[kMlpOut * kMlpH + t] = s;
 }
 
-// The row ranges of a batch of B: for the 256 x 256 layers sixteen of at least 64 rows
-// (their 32 tiles times the ranges fill the device twice or three times), for the
-// output layer 32 rows each.
-struct Ranges {
-    int per, per3 = 32;
-    size_t n, n3;
-    explicit Ranges(int B)
-        : per(std::max(64, ((B + 15) / 16 + kTileK - 1) / kTileK * kTileK)),
-          n((size_t)(B + per - 1) / per),
-          n3((size_t)(B + 31) / 32) {}
-};
-
 // The sums over the ranges into the gradients (layer 0 and 1: weights and biases; 2).
 __global__ void __launch_bounds__(256) k_sum_parts(const float* __restrict__ part, const float* __restrict__ part3,
                                                    int ranges, int ranges3, float* __restrict__ w0, float* __restrict__ b0,
@@ -328,7 +317,7 @@ void Mlp::ensure_work(int B) {
     if (cap >= B) return;
     cap = B;
     const size_t b = (size_t)B;
-    const Ranges r(B);
+    const MostRanges r(B);
     Part* const parts[] = {&xn, &z1, &a1, &z2, &a2, &g1, &g2, &z3, &g3, &part, &part3};
     const size_t floats[] = {b * kMlpIn, b * kMlpH, b * kMlpH, b * kMlpH, b * kMlpH, b * kMlpH, b * kMlpH,
                              b * kMlpOut, b * kMlpOut, 2 * r.n * kPart, r.n3 * kPart3};
