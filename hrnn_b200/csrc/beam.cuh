@@ -705,19 +705,27 @@ __device__ void greedy_descent(const DevView& v, WarpSmem& s, int top, int stop,
 }
 
 // Number of td[0..n) that are not above x (the insertion point after equal
-// distances), for the lanes that ask: a search with three probes a round, four
-// rounds for 200 entries instead of eight dependent shared-memory reads.
+// distances; x is no NaN, which are above everything), for the lanes that ask: a
+// search with three probes a round, four rounds for 200 entries instead of eight
+// dependent shared-memory reads.
 __device__ __forceinline__ uint32_t insert_pos(const float* td, uint32_t n, float x) {
     uint32_t step = 1, pos = 0;
     while (step * 4 <= n) step *= 4;  // uniform: n is the warp's
     for (; step; step >>= 2) {
         const uint32_t i0 = pos + step - 1, i1 = i0 + step, i2 = i1 + step;
         const float t0 = td[min(i0, n - 1)], t1 = td[min(i1, n - 1)], t2 = td[min(i2, n - 1)];
-        const uint32_t c = (uint32_t)(i0 < n && !(t0 > x)) + (uint32_t)(i1 < n && !(t1 > x)) +
-                           (uint32_t)(i2 < n && !(t2 > x));
+        const uint32_t c = (uint32_t)(i0 < n && t0 <= x) + (uint32_t)(i1 < n && t1 <= x) +
+                           (uint32_t)(i2 < n && t2 <= x);
         pos += c * step;
     }
     return pos;
+}
+
+// A whole number that orders as the distance does (the INT8 form's may come out below
+// 0), NaN last.
+__device__ __forceinline__ int order_key(float d) {
+    const int b = (int)__float_as_uint(d);
+    return b ^ (b >> 31 & 0x7FFFFFFF);
 }
 
 // Inserts the scored neighbours of the lanes with `have` (d, id) into the beam:
@@ -738,6 +746,10 @@ __device__ __forceinline__ uint32_t insert_pos(const float* td, uint32_t n, floa
 // binary search per entry, and shuffle loops for both rankings, took about two
 // thirds of the 8,000 cycles an expansion of a lone query cost at ef = 200.)
 //
+// A NaN distance (a NaN in the query or the row) is farther than every number and as
+// far as another NaN, the order of the bits that the team search compares: it goes to
+// the end of the beam and never enters a full one.
+//
 // known(d, ok, id, pos) is called by the whole warp once the neighbours to insert are
 // known (lanes with ok), before the beam changes.  DEDUP: an id may come twice (two
 // parents sharing a neighbour that the lossy visited cache did not catch): the lowest
@@ -746,7 +758,8 @@ template <bool DEDUP = false, class F>
 __device__ __forceinline__ void beam_insert(WarpSmem& s, float d, uint32_t id, bool have, uint32_t EF, uint32_t& tsize,
                                             uint32_t& cursor, F&& known) {
     const int lane = threadIdx.x & 31;
-    bool ok = have && !(tsize >= EF && d >= s.td[EF - 1]);
+    const bool nan = d != d;
+    bool ok = have && !(tsize >= EF && (nan || d >= s.td[EF - 1]));
     uint32_t pos = 0, ab = __ballot_sync(0xFFFFFFFFu, ok);
     if (ab) {
         if constexpr (DEDUP) {
@@ -754,8 +767,9 @@ __device__ __forceinline__ void beam_insert(WarpSmem& s, float d, uint32_t id, b
             if (ok && (same & lanemask_lt() & ab)) ok = false;
         }
         pos = insert_pos(s.td, tsize, d);
+        if (nan) pos = tsize;
         if (ok) {
-            for (int k = (int)pos - 1; k >= 0 && s.td[k] == d; --k)
+            for (int k = (int)pos - 1; k >= 0 && __float_as_uint(s.td[k]) == __float_as_uint(d); --k)
                 if (((s.ti[k] ^ id) & kIdMask) == 0) {
                     ok = false;
                     break;
@@ -769,14 +783,16 @@ __device__ __forceinline__ void beam_insert(WarpSmem& s, float d, uint32_t id, b
     // ranks among the accepted ones, then their insertion points in that order, four
     // at a time from shared memory (s.nd has been read: the callers hold d in registers)
     const bool pad = (uint32_t)lane >= na && (uint32_t)lane < ((na + 3) & ~3u);
-    if (ok) s.nd[me] = d;
-    if (pad) s.nd[lane] = __uint_as_float(0x7F800000u);
+    const int key = order_key(d);
+    int* const nk = reinterpret_cast<int*>(s.nd);
+    if (ok) nk[me] = key;
+    if (pad) nk[lane] = 0x7FFFFFFF;
     __syncwarp();
     uint32_t before = 0;
     for (uint32_t i = 0; i < na; i += 4) {
-        const float4 o = *reinterpret_cast<const float4*>(s.nd + i);
-        before += (uint32_t)(o.x < d || (o.x == d && i < me)) + (uint32_t)(o.y < d || (o.y == d && i + 1 < me)) +
-                  (uint32_t)(o.z < d || (o.z == d && i + 2 < me)) + (uint32_t)(o.w < d || (o.w == d && i + 3 < me));
+        const int4 o = *reinterpret_cast<const int4*>(nk + i);
+        before += (uint32_t)(o.x < key || (o.x == key && i < me)) + (uint32_t)(o.y < key || (o.y == key && i + 1 < me)) +
+                  (uint32_t)(o.z < key || (o.z == key && i + 2 < me)) + (uint32_t)(o.w < key || (o.w == key && i + 3 < me));
     }
     if (ok) s.apos[before] = pos;
     if (pad) s.apos[lane] = 0xFFFFFFFFu;
@@ -844,13 +860,14 @@ __device__ __forceinline__ uint32_t first_unexpanded(const WarpSmem& s, uint32_t
 // the neighbours of the one just expanded that are about to be inserted (lanes with
 // ok: distance d, insertion point pos) and the unexpanded beam entry after it
 // (`after` at `at`; kInvalid: none): the closest of them, the beam's at equal
-// distance.  None of the inserted ones then lands before it.
+// distance.  None of the inserted ones then lands before it, and it lands in the beam:
+// in a full one the neighbours with ok are closer than the last entry.
 __device__ __forceinline__ uint32_t next_entry(const WarpSmem& s, float d, bool ok, uint32_t id, uint32_t pos,
                                                uint32_t after, uint32_t& at) {
-    // distances are >= 0: their bits order as they do (a NaN is never the smallest)
+    // distances are >= 0 or NaN: their bits order as they do, NaN last
     const uint32_t best = __reduce_min_sync(0xFFFFFFFFu, ok ? __float_as_uint(d) : 0xFFFFFFFFu);
     const uint32_t have = __ballot_sync(0xFFFFFFFFu, ok && __float_as_uint(d) == best);
-    if (!have || (after != kInvalid && !(__uint_as_float(best) < s.td[at]))) return after;
+    if (!have || (after != kInvalid && best >= __float_as_uint(s.td[at]))) return after;
     const int i = __ffs(have) - 1;
     at = __shfl_sync(0xFFFFFFFFu, pos, i);
     return __shfl_sync(0xFFFFFFFFu, id, i);
@@ -879,12 +896,14 @@ __device__ uint32_t beam_search(const DevView& v, WarpSmem& s, uint32_t ep, floa
     // (next_entry) where a link row is a single load, else found by a scan.
     uint32_t c = ep, found = 0, row0 = 0, row1 = 0;
     if (short_rows) load_row(v, c, level, row0, row1);
-    while (c != kInvalid) {
+    // (no node is expanded twice, so v.n steps always do)
+    uint32_t steps = 0;
+    while (c != kInvalid && steps < v.n) {
         if (lane == 0) s.ti[found] = c | kExpanded;
         cursor = found + 1;
         uint32_t at = 0, after = kInvalid;
         if (short_rows) after = first_unexpanded(s, cursor, tsize, at);
-        c_exp++;
+        steps++;
         const uint32_t* adj = links_of(v, c, level);
         if (!short_rows) row0 = adj[0];
         const uint32_t size = __shfl_sync(0xFFFFFFFFu, row0, 0) & 0xFFFFu;
@@ -931,6 +950,7 @@ __device__ uint32_t beam_search(const DevView& v, WarpSmem& s, uint32_t ep, floa
             found = at;
         }
     }
+    c_exp += steps;
     return tsize;
 }
 
