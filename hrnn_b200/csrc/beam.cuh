@@ -687,7 +687,8 @@ __device__ void greedy_descent(const DevView& v, WarpSmem& s, int top, int stop,
                 __syncwarp();
                 warp_dist_list<DM, RK>(v, s.q, s.ni, cnt, s.nd);
                 c_dist += cnt;
-                float d = (uint32_t)lane < cnt ? s.nd[lane] : FLT_MAX;
+                // (idle lanes: no improvement even where the distances so far are infinite)
+                float d = (uint32_t)lane < cnt ? s.nd[lane] : __uint_as_float(0x7F800000u);
                 float mn = d;
                 for (int o = 16; o; o >>= 1) mn = fminf(mn, __shfl_xor_sync(0xFFFFFFFFu, mn, o));
                 uint32_t hit = __ballot_sync(0xFFFFFFFFu, (uint32_t)lane < cnt && d == mn);

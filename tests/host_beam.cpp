@@ -218,6 +218,52 @@ int fast_search(const Graph& g, float q, uint32_t EF, uint32_t vc) {
     return 0;
 }
 
+// The descent through two upper levels of a random graph, lists of `deg` links.
+int descent(uint32_t n, uint32_t deg, const std::vector<float>& values, float finite, float q) {
+    Graph g(n, 16, values, finite);
+    std::vector<uint32_t> up;
+    std::vector<uint64_t> off(n);
+    for (uint32_t i = 0; i < n; ++i) {
+        off[i] = up.size();
+        for (int level = 0; level < 2; ++level) {
+            up.push_back(pick(8) ? deg : pick(deg + 1));
+            for (uint32_t j = 0; j < deg; ++j) up.push_back(pick(n));
+        }
+    }
+    g.v.upper = up.data();
+    g.v.upper_off = off.data();
+    g.v.WU = deg + 1;
+    auto dist = [&](uint32_t i) { return (q - g.x[i]) * (q - g.x[i]); };
+    uint32_t want = 0;
+    for (int level = 2; level > 0; --level)
+        for (bool moved = true; moved;) {
+            moved = false;
+            const uint32_t* row = &up[off[want] + (size_t)(level - 1) * (deg + 1)];
+            uint32_t best = want;
+            for (uint32_t j = 0; j < row[0]; ++j)
+                if (dist(row[1 + j]) < dist(best)) {
+                    best = row[1 + j];
+                    moved = true;
+                }
+            want = best;
+        }
+    WarpSmem s = carve(smem(), 1, 32, 256);
+    s.q[0] = q;
+    uint32_t got[32];
+    if (!hostwarp::run(
+            [&] {
+                unsigned long long nd = 0;
+                uint32_t cur = 0;
+                float curd = dist(0);
+                greedy_descent<0, kRowsAny>(g.v, s, 2, 0, cur, curd, nd);
+                got[threadIdx.x] = cur;
+            },
+            1000000))
+        return std::printf("a descent does not end\n"), 1;
+    if (got[0] != want) return std::printf("descent to %u, not %u (query %g)\n", got[0], want, q), 1;
+    return 0;
+}
+
 }  // namespace
 
 int main() {
@@ -243,5 +289,10 @@ int main() {
                         for (float q : {0.f, 2.5f, kNan})
                             if (!r) r = exact_search(g, q, EF, vc) || (deg <= 32 && fast_search(g, q, EF, vc));
             }
+    for (const auto& k : kinds)
+        for (float finite : {0.f, .5f, 1.f})
+            for (uint32_t deg : {3u, 16u, 32u, 40u})
+                for (float q : {0.f, 2.5f, kNan, kInf, 1e30f})
+                    if (!r) r = descent(300, deg, k, finite, q);
     return r;
 }
