@@ -705,6 +705,22 @@ __device__ void greedy_descent(const DevView& v, WarpSmem& s, int top, int stop,
     }
 }
 
+// keys[0..n) = the n candidates (distinct ids) by (distance, id): distance bits << 32 |
+// id.  The distances are >= 0 or NaN, so their bits order as they do and a NaN has a
+// place of its own, last.
+__device__ __forceinline__ void order_candidates(const uint32_t* id, const float* d, uint32_t n, uint64_t* keys) {
+    for (uint32_t x = threadIdx.x & 31; x < n; x += 32) {
+        const uint32_t dx = __float_as_uint(d[x]), ix = id[x];
+        uint32_t r = 0;
+        for (uint32_t y = 0; y < n; ++y) {
+            const uint32_t dy = __float_as_uint(d[y]);
+            r += (dy < dx) || (dy == dx && id[y] < ix);
+        }
+        keys[r] = ((uint64_t)dx << 32) | ix;
+    }
+    __syncwarp();
+}
+
 // Number of td[0..n) that are not above x (the insertion point after equal
 // distances; x is no NaN, which are above everything), for the lanes that ask: a
 // search with three probes a round, four rounds for 200 entries instead of eight

@@ -400,16 +400,7 @@ __global__ void __launch_bounds__(128, 4) k_link_update(DevView v, LinkTable lt,
             __syncwarp();
         }
         const uint32_t total = c0 + nn;
-        for (uint32_t x = lane; x < total; x += 32) {
-            float dx = cd[x];
-            uint32_t ix_ = cid[x], r = 0;
-            for (uint32_t y = 0; y < total; ++y) {
-                float dy = cd[y];
-                r += (dy < dx) || (dy == dx && cid[y] < ix_);
-            }
-            keys[r] = ((uint64_t)__float_as_uint(dx) << 32) | ix_;
-        }
-        __syncwarp();
+        order_candidates(cid, cd, total, keys);
         for (uint32_t x = lane; x < total; x += 32) {
             cid[x] = (uint32_t)keys[x];
             cd[x] = __uint_as_float((uint32_t)(keys[x] >> 32));

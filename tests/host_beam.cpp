@@ -264,6 +264,28 @@ int descent(uint32_t n, uint32_t deg, const std::vector<float>& values, float fi
     return 0;
 }
 
+// A link list's candidates by (distance, id).
+int candidates(uint32_t n, const std::vector<float>& values) {
+    std::vector<uint32_t> id(n);
+    std::vector<float> d(n);
+    for (uint32_t i = 0; i < n; ++i) {
+        id[i] = (i * 7919u) % 4099u;
+        d[i] = values[pick((unsigned)values.size())];
+    }
+    std::vector<uint32_t> at(n);
+    for (uint32_t i = 0; i < n; ++i) at[i] = i;
+    std::sort(at.begin(), at.end(), [&](uint32_t a, uint32_t b) {
+        return nearer(d[a], d[b]) || (same(d[a], d[b]) && id[a] < id[b]);
+    });
+    std::vector<uint64_t> keys(n, ~0ull);
+    if (!hostwarp::run([&] { order_candidates(id.data(), d.data(), n, keys.data()); }, 1000))
+        return std::printf("an ordering does not end\n"), 1;
+    for (uint32_t i = 0; i < n; ++i)
+        if ((uint32_t)keys[i] != id[at[i]] || !same(__uint_as_float((uint32_t)(keys[i] >> 32)), d[at[i]]))
+            return std::printf("candidate %u of %u: %u, not %u\n", i, n, (uint32_t)keys[i], id[at[i]]), 1;
+    return 0;
+}
+
 }  // namespace
 
 int main() {
@@ -289,6 +311,9 @@ int main() {
                         for (float q : {0.f, 2.5f, kNan})
                             if (!r) r = exact_search(g, q, EF, vc) || (deg <= 32 && fast_search(g, q, EF, vc));
             }
+    for (const auto& k : kinds)
+        for (uint32_t n : {1u, 17u, 33u, 300u})
+            if (!r) r = candidates(n, k);
     for (const auto& k : kinds)
         for (float finite : {0.f, .5f, 1.f})
             for (uint32_t deg : {3u, 16u, 32u, 40u})
