@@ -16,6 +16,7 @@
 //   the reference's (hrnn.h:2055).
 // A query whose table or accepted list overflows is flagged and answered by the
 // global-memory warp kernel instead.
+#include <algorithm>
 #include <cfloat>
 #include <type_traits>
 
@@ -59,12 +60,14 @@ __global__ void k_kdist_column(DevView v, uint32_t kidx, float* __restrict__ kco
 __host__ __device__ constexpr uint32_t table_max(bool, bool) { return 8192; }
 
 // dynamic shared memory: q[dim] | keys[H] | cnt[H] (threshold > 1 only) |
-// stage[warps][64] | acc[kACap] | dists[warps][32] | ctl[16] | q8 (dim bytes, padded to 16) | qm,
-// H = table_max(counts, mixed)
+// stage[warps][64] | acc[kACap] | ctl[16] | q8 (dim bytes, padded to 16) | qm,
+// H = table_max(counts, mixed).  The exact forms, which have no q8, keep their warps'
+// distances in its place: dists[warps][32].
 __host__ size_t bc_cta_smem(uint32_t dim, bool counts, bool mixed) {
-    const size_t H = table_max(counts, mixed);
-    return (size_t)dim * 4 + H * 4 + (counts ? H * 4 : 0) + (kBCThreads / 32) * 96 * 4 + (size_t)kACap * 4 + 64 +
-           (((size_t)dim + 15) & ~(size_t)15) + 16;
+    const size_t H = table_max(counts, mixed), NW = kBCThreads / 32;
+    const size_t tail = (((size_t)dim + 15) & ~(size_t)15) + 16;
+    return (size_t)dim * 4 + H * 4 + (counts ? H * 4 : 0) + NW * 64 * 4 + (size_t)kACap * 4 + 64 +
+           (mixed ? tail : std::max(tail, NW * 32 * 4));
 }
 
 constexpr float kTieUlps = 16.f;  // FP64 re-decision band around the radius, in ulps of kd
@@ -87,8 +90,8 @@ __global__ void __launch_bounds__(kBCThreads) k_phase_bc_cta(
     uint32_t* cnt = keys + HM;
     uint32_t* stage = COUNTS ? cnt + HM : cnt;
     uint32_t* acc = stage + NW * 64;
-    float* dists = (float*)(acc + kACap);  // a warp's distances
-    uint32_t* ctl = (uint32_t*)(dists + NW * 32);  // 0: query, 1: accepted count, 2: overflow, 3: table full
+    uint32_t* ctl = acc + kACap;  // 0: query, 1: accepted count, 2: overflow, 3: table full
+    float* dists = (float*)(ctl + 16);  // exact forms: the warps' distances
     int* q8 = (int*)(ctl + 16);   // INT8 screen: the query as packed int8 words
     float4* qm = (float4*)((char*)q8 + ((v.dim + 15) & ~15u));  // (s_q^2 sum q8^2, s_q, ||q - s_q q8||, 0)
     const bool i8s = MIXED && v.i8_screen && v.vec_i8 != nullptr;
