@@ -26,6 +26,7 @@ struct Error : std::runtime_error {
 
 inline void cuda_check(cudaError_t e, const char* what, const char* file, int line) {
     if (e != cudaSuccess) {
+        cudaGetLastError();  // reported here: no later launch check is to find it
         char buf[512];
         std::snprintf(buf, sizeof(buf), "%s: %s (%s:%d)", what, cudaGetErrorString(e), file, line);
         fail(e == cudaErrorMemoryAllocation ? HRNN_ERR_NOMEM : HRNN_ERR_CUDA, buf);
