@@ -315,7 +315,7 @@ void Mlp::init(uint64_t seed, cudaStream_t s) {
 
 void Mlp::ensure_work(int B) {
     if (cap >= B) return;
-    cap = B;
+    cap = 0;  // until the parts stand: an allocation that fails has freed the former one
     const size_t b = (size_t)B;
     const MostRanges r(B);
     Part* const parts[] = {&xn, &z1, &a1, &z2, &a2, &g1, &g2, &z3, &g3, &part, &part3};
@@ -329,6 +329,7 @@ void Mlp::ensure_work(int B) {
         parts[i]->p = work.as<float>() + at;
         at += (floats[i] + 63) & ~(size_t)63;
     }
+    cap = B;
 }
 
 void Mlp::forward(const float* X, int B, cudaStream_t s) {
