@@ -43,10 +43,14 @@ DevView make_view(Index& ix);
 namespace {
 
 // Reverse links asked for by a batch, by target list (`key`: node id for level 0,
-// cap + upper block index above).  The first kSlots of a list sit in the list's own
-// 32-byte record; further ones (lists of hub points) in an overflow array, chained
-// from the list's head.  The new points are sorted before they are used, so the
-// order of arrival does not matter, and no grouping pass is needed.
+// cap + upper block index above).  Every link has a number of its own below maxreq; the
+// first to come to a list gives it its record, so only 8 bytes per list are needed
+// (40 with a record per list: 320 MB for one point inserted into an index with room for
+// 8M).  The first kSlots of a list sit in its record; further ones (lists of hub points)
+// are chained from the record's head, each in its number's place.  The new points are
+// sorted before they are used, so no grouping pass is needed, and the order of arrival
+// matters only for a list with more than kGroupMax links of one batch: it decides which
+// of them are applied, the others are dropped.
 struct Link {
     uint32_t src;     // new point
     float d;          // L2(new point, target)
@@ -56,13 +60,20 @@ struct OverLink {
     Link l;
     uint32_t next;    // kInvalid ends the chain
 };
+struct ListLinks {
+    uint32_t cnt;     // links asked for
+    uint32_t rec;     // 1 + the list's record (0: none yet)
+};
+struct ActiveList {
+    uint32_t key, target, rec;  // target: the node the list is of
+};
 struct LinkTable {
-    uint32_t* cnt;        // [keys] links asked for (0 between batches)
-    uint32_t* head;       // [keys] first overflow entry (kInvalid between batches)
-    Link* slot;           // [keys][kSlots]
-    OverLink* over;       // overflow entries of the batch
-    uint2* active;        // (key, target node) of the lists with new links
-    uint32_t* ctr;        // this batch's counters: active lists, overflow entries
+    ListLinks* list;      // [keys] zeros between batches
+    uint32_t* head;       // [maxreq] a record's latest chained link (kInvalid between batches)
+    Link* slot;           // [maxreq][kSlots]
+    OverLink* over;       // [maxreq]
+    ActiveList* active;   // [maxreq] the lists with new links
+    uint32_t* ctr;        // this batch's counters: active lists, links above level 0
 };
 
 constexpr uint32_t kMaxSel = 64;      // M of the heuristic (maxM0 for reverse pruning)
@@ -281,18 +292,20 @@ __global__ void __launch_bounds__(T == 1 ? 128 : 32 * T, T == 1 ? 4 : 2) k_build
             for (uint32_t i = lane; i < ns; i += 32) own[1 + i] = sel_id[ns - 1 - i];  // farthest first
             if (lane == 0) own[0] = ns;
             // the links back
+            uint32_t o0 = (p - b0) * M;  // this point's first number; above level 0 after all points'
+            if (level > 0) {
+                if (lane == 0) o0 = (b1 - b0) * M + atomicAdd(&lt.ctr[1], ns);
+                o0 = __shfl_sync(0xFFFFFFFFu, o0, 0);
+            }
             for (uint32_t i = lane; i < ns; i += 32) {
-                const uint32_t t = sel_id[i];
+                const uint32_t t = sel_id[i], o = o0 + i;
                 const uint32_t key = level == 0 ? t : cap + (uint32_t)(v.upper_off[t] / v.WU) + (uint32_t)(level - 1);
-                const uint32_t at = atomicAdd(&lt.cnt[key], 1u);
+                const uint32_t at = atomicAdd(&lt.list[key].cnt, 1u), had = atomicCAS(&lt.list[key].rec, 0u, o + 1);
+                const uint32_t rec = had ? had - 1 : o;
                 const Link l{p, sel_d[i]};
-                if (at == 0) lt.active[atomicAdd(&lt.ctr[0], 1u)] = make_uint2(key, t);
-                if (at < kSlots) {
-                    lt.slot[(size_t)key * kSlots + at] = l;
-                } else {
-                    const uint32_t o = atomicAdd(&lt.ctr[1], 1u);
-                    lt.over[o] = OverLink{l, atomicExch(&lt.head[key], o)};
-                }
+                if (!had) lt.active[atomicAdd(&lt.ctr[0], 1u)] = ActiveList{key, t, rec};
+                if (at < kSlots) lt.slot[(size_t)rec * kSlots + at] = l;
+                else lt.over[o] = OverLink{l, atomicExch(&lt.head[rec], o)};
             }
             cur = sel_id[0];
             curd = sel_d[0];
@@ -328,8 +341,8 @@ __global__ void __launch_bounds__(128, 4) k_link_update(DevView v, LinkTable lt,
     float* tmpd = (float*)scratch;
     const uint32_t na = lt.ctr[0];
     for (uint32_t g = blockIdx.x * wpb + w; g < na; g += gridDim.x * wpb) {
-        const uint32_t key = lt.active[g].x, t = lt.active[g].y;
-        const uint32_t nn = min(lt.cnt[key], kGroupMax);
+        const uint32_t key = lt.active[g].key, t = lt.active[g].target, rec = lt.active[g].rec;
+        const uint32_t nn = min(lt.list[key].cnt, kGroupMax);
         const bool lvl0 = key < cap;
         uint32_t* list = lvl0 ? adj0 + (size_t)t * v.W0 : upper + (size_t)(key - cap) * v.WU;
         const uint32_t Mcur = lvl0 ? maxM0 : maxM;
@@ -340,7 +353,7 @@ __global__ void __launch_bounds__(128, 4) k_link_update(DevView v, LinkTable lt,
         for (uint32_t x = lane; x < P; x += 32) {
             uint64_t k = ~0ull;
             if (x < min(nn, kSlots)) {
-                const Link l = lt.slot[(size_t)key * kSlots + x];
+                const Link l = lt.slot[(size_t)rec * kSlots + x];
                 k = ((uint64_t)__float_as_uint(l.d) << 32) | l.src;
             }
             keys[x] = k;
@@ -348,17 +361,17 @@ __global__ void __launch_bounds__(128, 4) k_link_update(DevView v, LinkTable lt,
         if (nn > kSlots) {  // the overflow chain
             __syncwarp();
             if (lane == 0) {
-                uint32_t o = lt.head[key];
+                uint32_t o = lt.head[rec];
                 for (uint32_t x = kSlots; x < nn; ++x) {
                     const OverLink e = lt.over[o];
                     keys[x] = ((uint64_t)__float_as_uint(e.l.d) << 32) | e.l.src;
                     o = e.next;
                 }
-                lt.head[key] = kInvalid;
+                lt.head[rec] = kInvalid;
             }
         }
         __syncwarp();
-        if (lane == 0) lt.cnt[key] = 0;  // ready for the next batch
+        if (lane == 0) lt.list[key] = ListLinks{0u, 0u};  // ready for the next batch
         for (uint32_t kk = 2; kk <= P; kk <<= 1)
             for (uint32_t j = kk >> 1; j > 0; j >>= 1) {
                 __syncwarp();
@@ -485,18 +498,18 @@ void add_points(Index& ix, const float* data, const uint64_t* labels, size_t n_a
     // The link table and the batches' counters (two each).
     const uint32_t cap = (uint32_t)ix.max_elements;
     const size_t keyspace = cap + ix.upper.size() / (1 + ix.maxM) + 1;
-    DevMem kcnt, khead, kslot, kover, active, ctr;
-    kcnt.alloc(keyspace * 4);
-    khead.alloc(keyspace * 4);
-    kslot.alloc(keyspace * kSlots * sizeof(Link));
+    DevMem klist, khead, kslot, kover, active, ctr;
+    klist.alloc(keyspace * sizeof(ListLinks));
+    khead.alloc(maxreq * 4);
+    kslot.alloc(maxreq * kSlots * sizeof(Link));
     kover.alloc(maxreq * sizeof(OverLink));
-    active.alloc(maxreq * sizeof(uint2));
+    active.alloc(maxreq * sizeof(ActiveList));
     ctr.alloc(std::max<size_t>(batches.size(), 1) * 8);
-    CUDA_CHECK(cudaMemsetAsync(kcnt.p, 0, kcnt.bytes, s));
+    CUDA_CHECK(cudaMemsetAsync(klist.p, 0, klist.bytes, s));
     CUDA_CHECK(cudaMemsetAsync(khead.p, 0xFF, khead.bytes, s));
     CUDA_CHECK(cudaMemsetAsync(ctr.p, 0, ctr.bytes, s));
-    LinkTable lt{kcnt.as<uint32_t>(), khead.as<uint32_t>(), kslot.as<Link>(), kover.as<OverLink>(),
-                 active.as<uint2>(), nullptr};
+    LinkTable lt{klist.as<ListLinks>(), khead.as<uint32_t>(), kslot.as<Link>(), kover.as<OverLink>(),
+                 active.as<ActiveList>(), nullptr};
     const int nsm = nsm_of(ix.device);
     const bool fused = (ix.order.fused & 1) != 0;
     const uint32_t efc = (uint32_t)((ix.ef_construction + 31) & ~(size_t)31);
@@ -535,7 +548,7 @@ void add_points(Index& ix, const float* data, const uint64_t* labels, size_t n_a
         CUDA_CHECK(cudaFuncSetAttribute(kbt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)team_smem));
     CUDA_CHECK(cudaFuncSetAttribute(kl, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_l));
     // All batches are enqueued without waiting: a batch's sizes on the device
-    // (active lists, overflow entries) are read there.
+    // (active lists, links above level 0) are read there.
     for (size_t bi = 0; bi < batches.size(); ++bi) {
         const Batch& b = batches[bi];
         ix.cur = b.p1;  // view covers the batch (vectors); the graph does not reach it yet
