@@ -177,35 +177,23 @@ __device__ __forceinline__ void quad_step(float (&acc)[4], float4 q, float4 x) {
     acc[3] = sq_step(acc[3], q.w - x.w, FUSED);
 }
 
-// Distances of q to vec rows ids[0..cnt), dim = 16 NB: eight rows per group, G
-// groups of loads in flight.
-template <bool FUSED, int NB, int G>
+// Distances of q to vec rows ids[0..cnt), dim = 16 NB: eight rows at a time.
+template <bool FUSED, int NB>
 __device__ __forceinline__ void warp_l2_quads(const DevView& v, const float* q, const uint32_t* ids, uint32_t cnt,
                                               float* dout) {
     const int lane = threadIdx.x & 31, c = lane & 3, r = lane >> 2;
     const float4* q4 = reinterpret_cast<const float4*>(q) + c;
-    for (uint32_t b = 0; b < cnt; b += 8 * G) {
-        float4 x[G][NB];
+    for (uint32_t b = 0; b < cnt; b += 8) {
+        float4 x[NB];
+        const uint32_t t = b + r;
+        const float4* x4 = reinterpret_cast<const float4*>(v.vec + (size_t)ids[t < cnt ? t : b] * (16 * NB)) + c;
 #pragma unroll
-        for (int g = 0; g < G; ++g) {
-            if (g == 0 || b + 8 * g < cnt) {  // uniform over the warp
-                const uint32_t t = b + 8 * g + r;
-                const float4* x4 = reinterpret_cast<const float4*>(v.vec + (size_t)ids[t < cnt ? t : b] * (16 * NB)) + c;
+        for (int i = 0; i < NB; ++i) x[i] = __ldg(x4 + 4 * i);
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                for (int i = 0; i < NB; ++i) x[g][i] = __ldg(x4 + 4 * i);
-            }
-        }
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            if (g == 0 || b + 8 * g < cnt) {
-                float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                for (int i = 0; i < NB; ++i) quad_step<FUSED>(acc, q4[4 * i], x[g][i]);
-                const float d = quad_sum16(acc[0], acc[1], acc[2], acc[3]);
-                const uint32_t t = b + 8 * g + r;
-                if (c == 0 && t < cnt) dout[t] = d;
-            }
-        }
+        for (int i = 0; i < NB; ++i) quad_step<FUSED>(acc, q4[4 * i], x[i]);
+        const float d = quad_sum16(acc[0], acc[1], acc[2], acc[3]);
+        if (c == 0 && t < cnt) dout[t] = d;
     }
 }
 
@@ -328,7 +316,7 @@ __device__ __forceinline__ void warp_l2_list(const DevView& v, const float* q, c
         for (uint32_t t = threadIdx.x & 31; t < cnt; t += 32)
             dout[t] = l2_thread(q, v.vec + (size_t)ids[t] * v.dim, v.dim, v.lanes, v.fused);
     } else {
-        warp_l2_quads<FUSED, RK / 16, 1>(v, q, ids, cnt, dout);
+        warp_l2_quads<FUSED, RK / 16>(v, q, ids, cnt, dout);
     }
     __syncwarp();
 }

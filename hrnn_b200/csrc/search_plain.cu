@@ -600,12 +600,13 @@ using KPhaseAFast = void (*)(DevView, const float*, uint32_t, const uint32_t*, c
                              uint32_t, float*, uint32_t*, uint32_t, uint32_t*, float*, uint32_t*, int,
                              const uint32_t*);
 
-// The two-parent kernel of a distance mode and width.
+// The two-parent kernel of a distance mode and width (BF16 rows: 96, 128 or 256).
 static KPhaseAFast phase_a_fast(int dm, bool r2, uint32_t dim) {
     auto of = [&](auto rk) -> KPhaseAFast {
         constexpr int RK = decltype(rk)::value;
-        if (dm == 3) return r2 ? k_phase_a_fast<3, true, RK> : k_phase_a_fast<3, false, RK>;
-        return r2 ? k_phase_a_fast<2, true, RK> : k_phase_a_fast<2, false, RK>;
+        if constexpr (RK != 0)
+            if (dm == 2) return r2 ? k_phase_a_fast<2, true, RK> : k_phase_a_fast<2, false, RK>;
+        return r2 ? k_phase_a_fast<3, true, RK> : k_phase_a_fast<3, false, RK>;
     };
     switch (dim) {
         case 96: return of(std::integral_constant<int, 96>{});
