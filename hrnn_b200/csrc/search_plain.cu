@@ -83,16 +83,17 @@ namespace {
 // Blocks per SM the registers are cut to.  10,000 queries on 300k x 128: 4 blocks with
 // sixteen rows in flight per warp 5.52 ms; eight rows in flight and 4 blocks 4.99, 5
 // 4.58, 6 4.28, 8 4.90.  6 is best at 64, 96, 256 and 272 too; widths read by quads of
-// single elements spill there (6,000 queries at d = 100: 4 3.01 ms, 6 4.29).
-constexpr int phase_a_blocks(int rk, int t) {
-    return t == 1 ? (rk == kRows4 ? 4 : 6) : rk == 64 || rk == kRows4 ? 3 : 2;
+// single elements spill there (6,000 queries at d = 100: 4 3.01 ms, 6 4.29), and BF16
+// rows want their loads in flight.
+constexpr int phase_a_blocks(int dm, int rk, int t) {
+    return t == 1 ? (rk == kRows4 || dm == 2 ? 4 : 6) : rk == 64 || rk == kRows4 ? 3 : 2;
 }
 
 // T: warps per query.  1: a warp of its own for each query.  kTeamWarps (exact forms):
 // the block's warps search for one query (beam_search_team), for batches too small to
 // fill the device.
 template <int DM, int RK, int T>
-__global__ void __launch_bounds__(T == 1 ? 128 : 32 * T, phase_a_blocks(RK, T)) k_phase_a(DevView v, const float* __restrict__ Q, uint32_t nq,
+__global__ void __launch_bounds__(T == 1 ? 128 : 32 * T, phase_a_blocks(DM, RK, T)) k_phase_a(DevView v, const float* __restrict__ Q, uint32_t nq,
                                                  const uint32_t* __restrict__ qm, const uint32_t* __restrict__ qef,
                                                  uint32_t efc, uint32_t vc, uint32_t mmax,
                                                  uint32_t* __restrict__ prox, uint32_t* __restrict__ nprox,
@@ -583,10 +584,11 @@ static bool phase_a_team(bool fast, int dm, const DevView& v, size_t nq, uint32_
            rows_kind(v.dim, v.lanes) != kRowsAny && warp_smem_bytes(v.dim, efc, team_vis(efc)) + 256 <= 227 * 1024;
 }
 
-// The reference-order kernel of a distance mode and the view's rows.
+// The reference-order kernel of a distance mode and the view's rows (BF16 rows: 96, 128
+// or 256, by pairs of lanes).
 static KPhaseA phase_a_exact(int dm, const DevView& v, bool team) {
     if (dm == 3) return k_phase_a<3, kRowsAny, 1>;
-    if (dm == 2) return k_phase_a<2, kRowsAny, 1>;
+    if (dm == 2) return v.dim == 96 ? k_phase_a<2, 96, 1> : v.dim == 128 ? k_phase_a<2, 128, 1> : k_phase_a<2, 256, 1>;
     return with_rows(rows_kind(v.dim, v.lanes), [&](auto rk) -> KPhaseA {
         constexpr int RK = decltype(rk)::value;
         if constexpr (RK != kRowsAny)
