@@ -129,7 +129,7 @@ __device__ __forceinline__ void sort_segment(E* __restrict__ seg, uint32_t len, 
 // One warp per segment of up to kWarpSegMax entries, sorted in registers by (rank,
 // owner); longer ones are listed in `big`, and the largest power of two at or above
 // a listed length is kept in *max_p.  With 64-bit keys in shared memory the 200k
-// segments of a 200k x 100 graph took 757 us, 32-bit keys in registers take 122 us.
+// segments of a 200k x 100 graph took 757 us, 32-bit keys in registers take 123 us.
 template <class E>
 __global__ void __launch_bounds__(32 * kSegWarps) k_sort_segments(const uint64_t* __restrict__ off, size_t n,
                                                                   E* __restrict__ ent, uint32_t rb,

@@ -6,7 +6,8 @@
 // same rounding as the CUDA-core GEMM of mlp.cu) and the products accumulated in
 // FP32 in tensor memory.  One CTA of 512 threads per 128 x 64 output tile: at 4096 rows
 // that is 128 CTAs, and a layer is bound by staging and by the GELU epilogue, not by
-// the products (44 us with 128 threads on 128 x 256 tiles, 30 with 512 threads).
+// the products (44 us with 128 threads on 128 x 256 tiles, 30 with 512 threads, 13 with
+// 512 threads on 128 x 64).
 //
 //   1. warp 0 allocates 64 TMEM columns (a 128 x 64 FP32 accumulator);
 //   2. all threads stage A's tile (128 x 256) and 64 rows of W (64 x 256) as BF16 in the

@@ -193,8 +193,7 @@ __global__ void __launch_bounds__(kBCThreads) k_phase_bc_cta(
                 break;
             }
             // ---- phase C: verify the table's candidates ----
-            // Candidates are staged per warp until 32 are ready, then verified one
-            // row per lane (32 rows in flight per warp).
+            // Candidates are staged per warp until 32 are ready, then verified.
             uint32_t* st = stage + w * 64;
             float* dl = dists + w * 32;
             uint32_t ns = 0;
