@@ -56,3 +56,24 @@ def test_builds_with_nan_and_huge_points(tmp_path, monkeypatch, d, what):
         h.saveIndex(str(p))
         raw.append(p.read_bytes())
     assert raw[0] == raw[1]
+
+
+@pytest.mark.parametrize("prec", [H.PREC_BF16, H.PREC_INT8])
+@pytest.mark.parametrize("nq", [9, 900])  # one warp per block; four
+def test_reduced_precision_searches_with_nan_and_huge_queries(prec, nq):
+    d = 128
+    h = H.HRNN(d, 3000, 16, 60, 100, 24)
+    h.add_points(data.mixture(3000, d, 12, 1.0, 3, 3))
+    h.refineKNNG(2, 20)
+    h.buildRKNNG()
+    h.set_precision(prec)
+    Q = data.mixture(nq, d, 12, 1.0, 3, 77)
+    want = h.search_rknn_batch(Q, 5, 24, 200)
+    B = Q.copy()
+    B[1, 0] = np.nan
+    B[4] = np.nan
+    B[6, d - 1] = np.inf
+    B[7] = 1e30
+    got = h.search_rknn_batch(B, 5, 24, 200)
+    assert all(len(got[i]) == 0 for i in (1, 4, 6, 7))
+    assert all(np.array_equal(got[i], want[i]) for i in range(nq) if i not in (1, 4, 6, 7))
